@@ -17,21 +17,21 @@
 //      exactly, t_h - m exact by Sterbenz's lemma), and one Newton step in
 //      double-double gives cbrt(m) = z - res y^2 / 3 (y^2 = 1 / z^2 to working
 //      precision);
-//   4. ln(x), which enters the result scaled by 2^-54 / 3: first from a
-//      single-precision logarithm, which decides the rounding unless the
-//      value lies within 2^-70 of a midpoint between doubles (checked from
-//      the exact rounding error of the final sum); then, in those rare
-//      cases, as e' ln 2 + 2 atanh(s), s = (f' - 1) / (f' + 1), f' in
-//      [1/sqrt 2, sqrt 2), by its odd series (absolute error below 1e-15);
+//   4. ln(x), which enters the result scaled by 2^-54 / 3, as e' ln 2 +
+//      2 atanh(s), s = (f' - 1) / (f' + 1), f' in [1/sqrt 2, sqrt 2), by its
+//      odd series (absolute error below 1e-15);
 //   5. the double-double value times (1 - 2^-54 ln(x)/3) is rounded once to
 //      double and scaled by 2^q (exact).
 // The result differs from the correctly rounded x^c only when x^c lies within
 // about 2^-100 relative of a midpoint between two doubles.
 //
-// The single-precision logarithm only chooses between the two evaluations
-// of step 4 (the device's and the host's may differ; the result does not),
-// so the strict kernels and the oracle (which evaluates the same expression
-// as a correctly rounded pow) agree bit for bit.
+// Most depths take a shorter way (pow_third_near): steps 2-5 on x itself from
+// a single-precision start, with a rounding test that sends the values too
+// near a midpoint for its accuracy to the full method.  Both give the
+// correctly rounded value, so the device's and the host's single-precision
+// functions may differ and the result does not: the strict kernels and the
+// oracle (which evaluates the same expression as a correctly rounded pow)
+// agree bit for bit.
 #pragma once
 
 #include <cmath>
@@ -70,10 +70,14 @@ DGSWEM_HD double ln_series(double f, int e) {
   return (double)ep * ln2_hi + ((double)ep * ln2_lo + lnf);
 }
 
-// kFastLog = false takes the series for ln(x) every time (the rare path
-// alone, for tests).
-template <bool kFastLog = true>
-DGSWEM_HD double pow_third(double x) {
+// The method for every x (out of line: the kernels reach it once in 2^17
+// calls, or outside the range of pow_third_near).
+#if defined(__CUDACC__)
+inline __host__ __device__ __noinline__
+#else
+inline
+#endif
+double pow_third_any(double x) {
   if (!(x > 0.0) || !(x < INFINITY)) {
     // pow(x, c) of a zero, negative, infinite or NaN base: 0, NaN, inf, NaN
     if (x == 0.0) return 0.0;
@@ -103,35 +107,68 @@ DGSWEM_HD double pow_third(double x) {
   const double t_l = fma(p_h, z, -t_h);
   const double res = (t_h - m) + (t_l + p_l * z);
   const double corr = (res * y2) * third;  // cbrt(m) = z - corr
-  // steps 4-5, first with ln(x) from a single-precision logarithm (absolute
-  // error below 2^-20 for f in [0.5, 1)): delta is then known to 2^-75, and
-  // z + tail rounds to the same double as the exact value unless the exact
-  // value lies within 2^-70 (relative) of a midpoint between two doubles.
-  // s = RN(z + tail) and its rounding error err (exact, |tail| << z) show
-  // that distance: |err| far from half an ulp of s keeps s.  Otherwise --
-  // about once in 2^18 calls -- ln(x) to 1e-15 by its series.
   const double k54 = 5.5511151231257827e-17 * third;  // 2^-54 / 3
-  if (kFastLog) {
-#if defined(__CUDA_ARCH__)
-    const float lnf_fast = __logf((float)f);
-#else
-    const float lnf_fast = std::log((float)f);
-#endif
-    const double lnx_fast = (double)e * 0.69314718055994531 + (double)lnf_fast;
-    const double delta_fast = lnx_fast * k54;
-    const double tail_fast = (-corr - z * delta_fast) + corr * delta_fast;
-    const double s = z + tail_fast;
-    const double err = tail_fast - (s - z);
-    int es;
-    const double fs = frexp(s, &es);                // s = fs 2^es, fs in [0.5, 1)
-    const double half_ulp = ldexp(1.0, es - 54);    // half an ulp of s
-    if (fs != 0.5 && fabs(fabs(err) - half_ulp) > s * 0x1p-70) return ldexp(s, q);
-  }
-  // step 4-5 with ln(x) to 1e-15 (also when s is a power of two, whose ulp
-  // below is half the one above)
   const double delta = ln_series(f, e) * k54;
   const double tail = (-corr - z * delta) + corr * delta;
   return ldexp(z + tail, q);
+}
+
+// Steps 2-5 for x in [2^-30, 2^30] (every depth of a run), without the
+// scaling of step 1: started from l2 ~ log2(x), to 2^-17 absolute, and
+// y0 ~ x^(-1/3), to 2^-19 relative.  One cubically convergent step takes u =
+// x y0^2 to z ~ x^(1/3): with e = 1 - x y0^3 (below 2^-17), x^(1/3) =
+// u (1 - e)^(-2/3) = u (1 + 2/3 e + 5/9 e^2 + O(e^3)).  The residual and the
+// correction are those of step 3 (1 / z^2 as y0^2 (1 + 2/3 e), good to 2^-35,
+// which the correction's own size, 2^-51, takes to 2^-86), and ln(x) = l2
+// ln 2 is known to 2^-17.5, so z + tail has a relative error below 2^-72.
+// Rounding both z + tail - 2^-71 z and z + tail + 2^-71 z (Ziv's test): equal
+// values are the correctly rounded one (true); otherwise -- about once in
+// 2^17 calls -- the result is left to pow_third_any (false).
+DGSWEM_HD bool pow_third_near(double x, float l2, float y0f, double* out) {
+  const double y0 = (double)y0f;
+  const double u = x * y0 * y0;
+  const double e = fma(-u, y0, 1.0);
+  const double z = fma(u, e * fma(e, 5.0 / 9.0, 2.0 / 3.0), u);
+  const double p_h = z * z;
+  const double p_l = fma(z, z, -p_h);
+  const double t_h = p_h * z;
+  const double t_l = fma(p_h, z, -t_h);
+  const double res = (t_h - x) + fma(p_l, z, t_l);
+  const double w = (y0 * (1.0 / 3.0)) * y0;
+  const double corr = res * fma(w, e * (2.0 / 3.0), w);
+  const double delta = (double)(l2 * (0.69314718f * (5.5511151e-17f / 3.0f)));  // ln(x) 2^-54 / 3
+  const double tail = fma(-z, delta, -corr);
+  const double lo = z + fma(z, -0x1p-71, tail), hi = z + fma(z, 0x1p-71, tail);
+  *out = hi;
+  return lo == hi;
+}
+
+// pow_third_near with its start: the value, and whether it holds (x in range
+// and the rounding test passed)
+DGSWEM_HD bool pow_third_try(double x, double* out) {
+#if defined(__CUDA_ARCH__)
+  const float l2 = __log2f((float)x);
+  float y0;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(l2 * (-1.0f / 3.0f)));
+#else
+  const float l2 = std::log2((float)x), y0 = std::exp2(l2 * (-1.0f / 3.0f));
+#endif
+  const bool near = pow_third_near(x, l2, y0, out);
+  return near && x >= 0x1p-30 && x <= 0x1p30;
+}
+
+// DEPTH**(1.D0/3.D0), correctly rounded.  The start comes from the base-2
+// single-precision logarithm and exponential (on the device the approximate
+// instructions: lg2 within 2^-22 relative, so 30 * 2^-22 < 2^-17 here).
+// 24 double-precision operations where pow_third_any's five Newton steps,
+// frexp and ldexp take about 70 and three times as many integer ones: the
+// strict stage kernel's volume terms take 2,200 cycles a tile of 128 elements
+// now, 3,900 before.  kNear = false takes pow_third_any for every x (for tests).
+template <bool kNear = true>
+DGSWEM_HD double pow_third(double x) {
+  double r;
+  if (kNear && pow_third_try(x, &r)) return r;
+  return pow_third_any(x);
 }
 
 // x / 3, correctly rounded, without a division: q = RN(x t), t = RN(1/3);
@@ -150,5 +187,66 @@ DGSWEM_HD double div3(double x) {
   const double r = fma(-q, 3.0, x);
   return copysign(fma(r, t, q), x);
 }
+
+// ---- reciprocal, quotient and square root, correctly rounded -----------------
+// The IEEE results of 1 / x, a / b and sqrt(x) from a seed of about 20 bits, by
+// one step of cubic convergence and Markstein's final step (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990: the residual of a result within an ulp is exact in one fma, and a
+// second fma rounds the corrected result once).  For arguments in mid_range
+// only, where no intermediate under- or overflows; the caller tests the range
+// of all the values of a point at once and takes the operators for the rest,
+// instead of a test and a branch in every operation.
+//
+// Reciprocal: y0 = (1 - e0) / x, |e0| <= 2^-19.9.  y1 = y0 + y0 (e0 + e0^2) =
+// (1 - e0^3) / x up to one rounding: within 0.6 ulp.  e1 = 1 - x y1 is exact,
+// and y1 + y1 e1 = (1 - e1^2) / x, |e1| < 2^-52, is rounded once: the correct
+// rounding unless 1 / x lies above a midpoint by less than 2^-104 of itself,
+// that is 2^106 - M X = k for a 53-bit X, an odd 54-bit M and k <= 4.
+// Square root: with y0 ~ 1 / sqrt(a) to 2^-19.9, g0 = a y0, h0 = y0 / 2, r =
+// 1/2 - g0 h0, both are multiplied by 1 + r + 3/2 r^2 ((1 - 2r)^(-1/2) up to
+// 5/2 r^3); d = a - g1^2 is exact and g1 + d h1 lies within 2^-103 of sqrt(a),
+// so its rounding is correct unless sqrt(a) is that near a midpoint, M^2 - 4 A
+// = k (A the 53-bit mantissa times a power of two, M odd), |k| < 128.
+// The few arguments so near a midpoint are all listed and tested, with every
+// seed within the bounds, in tests/test_rounded_ops.py: only a significand of
+// all ones can be rounded wrongly, in both, and mid_range leaves it out.
+DGSWEM_HD double rcp_from(double x, double y0) {
+  const double e0 = fma(-x, y0, 1.0);
+  const double y1 = fma(y0, fma(e0, e0, e0), y0);
+  return fma(fma(-x, y1, 1.0), y1, y1);
+}
+// a / b with y = 1 / b correctly rounded (Markstein): q is within an ulp
+DGSWEM_HD double quot_from(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+DGSWEM_HD double sqrt_from(double a, double y0) {
+  const double g0 = a * y0, h0 = 0.5 * y0;
+  const double r = fma(-g0, h0, 0.5);
+  const double c = fma(1.5 * r, r, r);
+  const double g1 = fma(g0, c, g0), h1 = fma(h0, c, h0);
+  return fma(fma(-g1, g1, a), h1, g1);
+}
+
+#if defined(__CUDACC__)
+// positive, between 2^-256 and 2^256 and not all ones in the significand's low
+// word
+__device__ __forceinline__ bool mid_range(double x) {
+  return (unsigned)(__double2hiint(x) - 0x2ff00000) < 0x20000000u && __double2loint(x) != -1;
+}
+// seeds: the approximate instructions, which read the high 32 bits (relative
+// errors over every high word of two binades, measured: 2^-19.9 and 2^-20.0)
+__device__ __forceinline__ double rcp_seed(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rsqrt_seed(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+#endif
 
 }  // namespace dgswem

@@ -96,6 +96,30 @@ static BasisP1 make_basis_p1() {
       B.mw[k][i] = B.m_inv[k] * B.wagp[i];
       B.srfac[k][i] = B.m_inv[k] * B.wagp[i] * B.phi_area[k][i];
     }
+  // the stage kernel's tables (see BasisT): its sums and traces rely on the
+  // factors below being exact, and on mode 1 and the area weights being
+  // constants
+  bool ok = true;
+  const double w = B.edgeq[0][0][0];
+  for (int l = 0; l < 3; ++l)
+    for (int j = 0; j < 3; ++j) {
+      int ex;
+      for (int k = 1; k < 3; ++k) {
+        const double t = B.phi_edge[l][j][k];
+        B.tr[l][j][k - 1] = t;
+        ok = ok && (t == 0.0 || std::fabs(std::frexp(t, &ex)) == 0.5);
+      }
+      const double s1 = B.phi_edge[l][j][1] * (j == 1 ? 8.0 : 2.0), s2 = B.edgeq[l][j][2];
+      ok = ok && B.phi_edge[l][j][0] == 1.0 && B.edgeq[l][j][0] == (j == 1 ? 4.0 * w : w) &&
+           B.edgeq[l][j][1] == s1 * w && (s2 == 0.0 || std::fabs(std::frexp(s2, &ex)) == 0.5);
+      B.sw[1][l][j][0] = B.sw[0][l][2 - j][0] = s1;
+      B.sw[1][l][j][1] = B.sw[0][l][2 - j][1] = s2;
+    }
+  for (int i = 0; i < 3; ++i)
+    for (int k = 0; k < 3; ++k)
+      ok = ok && B.mw[k][i] == B.mw[k][0] && B.phi_area[0][i] == 1.0 && B.drphi[k][i] == (k == 2 ? 1.0 : 0.0) &&
+           B.dsphi[k][i] == (k == 0 ? 0.0 : k == 1 ? 1.5 : 0.5);
+  if (!ok) throw Failure(DGSWEM_ERR_ARG, "p=1 tables are not the powers of two the stage kernel takes them for");
   return B;
 }
 
@@ -272,6 +296,7 @@ struct Variant {
   unsigned real_bytes;
   void (*set_basis)(const BasisP1&);
   void (*stage)(const StageArgs&, bool, int, unsigned, size_t, cudaStream_t);
+  void (*task_normals)(const MeshView&, int, void*, unsigned, cudaStream_t);
   void (*ibarrier)(const StageArgs&, bool, cudaStream_t);
   void (*node_minmax)(const LimitArgs&, unsigned, cudaStream_t);
   void (*limit_wetdry)(const LimitArgs&, int, cudaStream_t);
@@ -283,15 +308,15 @@ struct Variant {
   void (*halo)(bool, double*, int*, int, const int*, int, int, double*, cudaStream_t);
 };
 
-static const Variant kFast = {8, fast::set_basis, fast::launch_stage, fast::launch_ibarrier, fast::launch_node_minmax,
+static const Variant kFast = {8, fast::set_basis, fast::launch_stage, fast::launch_task_normals, fast::launch_ibarrier, fast::launch_node_minmax,
                               fast::launch_limit_wetdry, fast::launch_modal2nodal,
                               fast::launch_fortran_to_soa, fast::launch_soa_to_fortran, fast::launch_gather_int,
                               fast::launch_halo};
-static const Variant kStrict = {8, strict::set_basis, strict::launch_stage, strict::launch_ibarrier, strict::launch_node_minmax,
+static const Variant kStrict = {8, strict::set_basis, strict::launch_stage, strict::launch_task_normals, strict::launch_ibarrier, strict::launch_node_minmax,
                                 strict::launch_limit_wetdry, strict::launch_modal2nodal,
                                 strict::launch_fortran_to_soa, strict::launch_soa_to_fortran,
                                 strict::launch_gather_int, strict::launch_halo};
-static const Variant kMixed = {4, mixed::set_basis, mixed::launch_stage, mixed::launch_ibarrier, mixed::launch_node_minmax,
+static const Variant kMixed = {4, mixed::set_basis, mixed::launch_stage, mixed::launch_task_normals, mixed::launch_ibarrier, mixed::launch_node_minmax,
                                mixed::launch_limit_wetdry, mixed::launch_modal2nodal,
                                mixed::launch_fortran_to_soa, mixed::launch_soa_to_fortran,
                                mixed::launch_gather_int, mixed::launch_halo};
@@ -351,7 +376,8 @@ struct dgswem_cuda {
   DevBuf<float> egeof;  // FP32 geometry rows of a mixed-precision handle
   DevBuf<int> nm, link, star_ptr, star, ib_elem, ib_led;
   DevBuf<unsigned> einfo, eslot, tile_tasks;
-  DevBuf<int> tile_elem_ptr, tile_task_ptr, tile_halo_ptr, tile_halo;
+  DevBuf<int> tile_count, tile_halo;
+  DevBuf<double> tile_nrm, xres;  // per task: its normal; the ex side's momentum fluxes where one side is dry
   int ntile = 0;
   // tiles that read no ghost element and no internal-barrier side first
   // (n_tile_interior of them), then the others: the stage can start on the
@@ -519,6 +545,15 @@ struct LaunchTimer {
 
 unsigned grid_for(int n, int block) { return (unsigned)((n + block - 1) / block); }
 
+// Normals of the plan's edge tasks from the geometry table (device).
+void fill_task_normals(dgswem_cuda* h) {
+  if (h->v2) return;
+  h->v->task_normals(h->mesh, kTileShapes[h->tile_shape].tile, h->tile_nrm.p, (unsigned)h->ntile, h->stream);
+  check_launch(h, "task_normals");
+  --h->launches;  // part of the plan, not of a step
+  DG_CUDA(cudaStreamSynchronize(h->stream));
+}
+
 // Stage tile plan of the handle's tile shape (h->tile_shape): for each tile
 // of consecutive elements, the edge tasks it evaluates and the out-of-tile
 // neighbours (halo) they read.  Edge ownership: a boundary edge of a listed
@@ -529,44 +564,17 @@ unsigned grid_for(int n, int block) { return (unsigned)((n + block - 1) / block)
 // element order, then the boundary kinds grouped, so that a warp's tasks
 // mostly take one branch.  Tiles cover the first n_tiled elements (the owned
 // ones); `ne` is the row stride of link (all local elements, ghosts
-// included).  Tiles are cut sequentially, then planned in parallel (each
-// writes only its own elements' eslot).
+// included).  Tiles are planned in parallel (each writes only its own
+// elements' eslot).
 void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>& link,
                      const std::vector<unsigned>& einfo) {
   const TileShape shape = kTileShapes[h->tile_shape];
-  // Tiles: consecutive elements, at most shape.tile of them and at most
-  // shape.threads edge tasks (one pass of the block over its tasks).  An
-  // element adds a task per listed boundary edge and per interior edge whose
-  // neighbour is not already in the tile.
-  std::vector<int> elem_ptr(1, 0);
-  {
-    int t0 = 0, count = 0;
-    for (int e = 0; e < n_tiled; ++e) {
-      int add = 0;
-      for (int l = 0; l < 3; ++l) {
-        const unsigned kind = ei_kind(einfo[e], l);
-        if (kind == kNone) continue;
-        if (kind == kInterior) {
-          const int nb = link[(size_t)l * ne + e];
-          if (nb >= t0 && nb < e) continue;
-        }
-        ++add;
-      }
-      if (e - t0 == shape.tile || count + add > shape.threads) {
-        elem_ptr.push_back(e);
-        t0 = e;
-        count = 0;
-        e -= 1;  // recount the element against the new tile
-        continue;
-      }
-      count += add;
-    }
-    elem_ptr.push_back(n_tiled);
-  }
-  const int ntile = (int)elem_ptr.size() - 1;
+  // tile t: elements t * shape.tile ..; at most 3 * shape.tile <= shape.threads tasks
+  const int ntile = (n_tiled + shape.tile - 1) / shape.tile;
   std::vector<std::vector<unsigned>> ttasks(ntile);  // (word, list) pairs per tile
   std::vector<std::vector<int>> thalo(ntile);
   std::vector<unsigned> eslot(ne, 0u);
+  std::vector<int> count(2 * (size_t)std::max(ntile, 1), 0);
   int max_halo = 0, max_tasks = 0;
   struct Task {
     unsigned word, list;
@@ -578,7 +586,7 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
     std::vector<Task> tt;
 #pragma omp for schedule(dynamic, 64) reduction(max : max_halo, max_tasks)
     for (int t = 0; t < ntile; ++t) {
-      const int t0 = elem_ptr[t], t1 = elem_ptr[t + 1];
+      const int t0 = t * shape.tile, t1 = std::min(t0 + shape.tile, n_tiled);
       hl.clear();
       for (int e = t0; e < t1; ++e)
         for (int l = 0; l < 3; ++l)
@@ -593,8 +601,10 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
         return (unsigned)(shape.tile + (std::lower_bound(hl.begin(), hl.end(), g) - hl.begin()));
       };
       tt.clear();
-      for (int pass = 0; pass < 2; ++pass)  // interior edges, then boundary kinds
-        for (unsigned want = pass == 0 ? (unsigned)kInterior : 1u; want <= (pass == 0 ? 0u : 6u); ++want)
+      // interior edges of two tile elements, those to a halo element, boundary kinds
+      for (int pass = 0; pass < 3; ++pass) {
+        if (pass == 1) count[2 * t + 1] = (int)tt.size();
+        for (unsigned want = pass < 2 ? (unsigned)kInterior : 1u; want <= (pass < 2 ? 0u : 6u); ++want)
           for (int e = t0; e < t1; ++e)
             for (int l = 0; l < 3; ++l) {
               const unsigned info = einfo[e], kind = ei_kind(info, l);
@@ -603,6 +613,7 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
               unsigned w = kind << TaskBits::kKind, list = 0;
               if (kind == kInterior) {
                 const bool local = lk >= t0 && lk < t1, in_side = ei_flag(info, l) != 0;
+                if (local != (pass == 0)) continue;
                 if (local && !in_side) continue;  // the in side's task
                 const unsigned nled = ei_nled(info, l);
                 if (in_side)
@@ -617,6 +628,8 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
               }
               tt.push_back({w, list, e, l});
             }
+      }
+      count[2 * t] = (int)tt.size();
       for (int e = t0; e < t1; ++e) eslot[e] = kNoTask | kNoTask << 10 | kNoTask << 20;
       auto set_slot = [&](int e, int l, unsigned ti) {
         eslot[e] = (eslot[e] & ~(kNoTask << (10 * l))) | ti << (10 * l);
@@ -641,25 +654,23 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
       max_tasks = std::max(max_tasks, (int)tt.size());
     }
   }
+  max_halo = std::max(max_halo, 1);  // strides of the plan's arrays
+  max_tasks = std::max(max_tasks, 1);
   if (max_halo + shape.tile > kMaxTileSlots || max_tasks >= (int)kNoTask)
     throw Failure(DGSWEM_ERR_ARG, "stage tile plan exceeds the task word's slot range");
-  const size_t stage_smem = stage_layout(shape.tile, max_halo, std::max(max_tasks, 1), h->v->real_bytes).bytes;
+  const size_t stage_smem = stage_layout(shape.tile, max_halo, max_tasks, h->v->real_bytes).bytes;
   int dev_smem = 0;
   DG_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
   if (stage_smem > (size_t)dev_smem)
     throw Failure(DGSWEM_ERR_ARG, "stage tile needs " + std::to_string(stage_smem) +
                                       " bytes of shared memory, the device allows " + std::to_string(dev_smem));
-  std::vector<int> task_ptr(ntile + 1, 0), halo_ptr(ntile + 1, 0), halo;
-  std::vector<unsigned> tasks;
+  const size_t nt = (size_t)std::max(ntile, 1);
+  std::vector<unsigned> tasks(2 * nt * max_tasks, 0u);
+  std::vector<int> halo(nt * max_halo, -1);
+#pragma omp parallel for schedule(static)
   for (int t = 0; t < ntile; ++t) {
-    task_ptr[t + 1] = task_ptr[t] + (int)ttasks[t].size() / 2;
-    halo_ptr[t + 1] = halo_ptr[t] + (int)thalo[t].size();
-  }
-  tasks.reserve(2 * (size_t)task_ptr[ntile]);
-  halo.reserve((size_t)halo_ptr[ntile]);
-  for (int t = 0; t < ntile; ++t) {
-    tasks.insert(tasks.end(), ttasks[t].begin(), ttasks[t].end());
-    halo.insert(halo.end(), thalo[t].begin(), thalo[t].end());
+    std::copy(ttasks[t].begin(), ttasks[t].end(), tasks.begin() + 2 * (size_t)t * max_tasks);
+    std::copy(thalo[t].begin(), thalo[t].end(), halo.begin() + (size_t)t * max_halo);
   }
   {
     std::vector<int> order, rest;
@@ -675,22 +686,25 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
     h->tile_order.upload(order.empty() ? std::vector<int>(1, 0) : order);
   }
   h->ntile = ntile;
-  h->tile_elem_ptr.upload(elem_ptr);
-  h->tile_task_ptr.upload(task_ptr);
-  h->tile_halo_ptr.upload(halo_ptr);
-  h->tile_tasks.upload(tasks.empty() ? std::vector<unsigned>(2, 0u) : tasks);
-  h->tile_halo.upload(halo.empty() ? std::vector<int>(1, 0) : halo);
+  h->tile_count.upload(count);
+  h->tile_tasks.upload(tasks);
+  h->tile_halo.upload(halo);
   h->eslot.upload(eslot);
   h->stage_smem = stage_smem;
   MeshView& m = h->mesh;
   m.max_halo = max_halo;
   m.max_tasks = max_tasks;
-  m.tile_elem_ptr = h->tile_elem_ptr.p;
-  m.tile_task_ptr = h->tile_task_ptr.p;
+  m.ne_tiled = n_tiled;
+  m.tile_count = reinterpret_cast<const int2*>(h->tile_count.p);
   m.tile_tasks = reinterpret_cast<const uint2*>(h->tile_tasks.p);
-  m.tile_halo_ptr = h->tile_halo_ptr.p;
   m.tile_halo = h->tile_halo.p;
   m.eslot = h->eslot.p;
+  if (!h->v2) {
+    h->tile_nrm.alloc(2 * nt * max_tasks);
+    h->xres.alloc(6 * nt * max_tasks);
+    m.tile_nrm = h->tile_nrm.p;
+    if (m.egeo) fill_task_normals(h);  // a new plan of a built mesh
+  }
 }
 
 // Device element and node order: elements sorted along a Morton (Z-order)
@@ -979,6 +993,7 @@ void build_layout(dgswem_cuda* h, const dgswem_cuda_setup* s, const PartPlan& pl
   m.ebht = h->ebht.p; m.ebcfsp = h->ebcfsp.p;
   m.ib_elem = h->ib_elem.p; m.ib_led = h->ib_led.p;
   m.ibht = h->ibht.p; m.ibcfsb = h->ibcfsb.p; m.ibcfsp = h->ibcfsp.p;
+  fill_task_normals(h);
 }
 
 // Halo index lists of a partitioned handle (local element ids), per kind,
@@ -1145,6 +1160,14 @@ void launch_stage_rhs(dgswem_cuda* h, int it, int irk, const double* forcing, co
     A.b[I - 1] = h->btvd[(size_t)(irk - 1) * nrk + (I - 1)] * h->dtdp;
   }
   A.rout = h->keep_rhs[irk - 1] ? h->rhs[irk - 1].p : nullptr;
+  A.ca0 = A.a[0];
+  A.ca = A.a[irk - 1];
+  A.cb = A.b[irk - 1];
+  {
+    bool two = irk > 1 && A.a[0] != 0.0 && A.b[0] == 0.0;
+    for (int I = 1; I < irk - 1; ++I) two = two && A.a[I] == 0.0 && A.b[I] == 0.0;
+    A.ssp = A.ca == 0.0 || A.cb == 0.0 ? kSspAny : irk == 1 ? kSspOne : two ? kSspTwo : kSspAny;
+  }
   A.wd = h->wd.p;
   stage_clock(h, it, irk, &A.timedg, &A.rampdg);
   A.ramp = ramp;
@@ -1154,6 +1177,7 @@ void launch_stage_rhs(dgswem_cuda* h, int it, int irk, const double* forcing, co
   A.wsy = h->wsy.p;
   A.pr = h->pr.p;
   A.ib_rhs = h->ib_rhs.p;
+  A.xres = h->xres.p;
   A.err = h->err.p;
   const bool nonlin = h->ph.nleq == 1.0 && h->ph.leq == 0.0;
   if (h->mesh.nibseg > 0 && set != kInteriorTiles) {  // interior tiles have no barrier sides

@@ -11,7 +11,8 @@
 //   einfo[e]           packed edge kinds, processing order, orientation bits
 //   hb[k*NE + e]       bathymetry modes HB(k,e)
 //   stage tile plan    per tile of consecutive elements (TileShape): its edge tasks
-//                      (uint2 each, interior edges first, then boundary kinds)
+//                      (uint2 each: interior edges of two tile elements, of a tile
+//                      and a halo element, then boundary kinds)
 //                      and its halo (out-of-tile neighbours, global ids);
 //                      eslot[e] names the task of each local edge
 // Geometry (areas, Jacobian, edge lengths and normals) is recomputed from the
@@ -61,6 +62,12 @@ struct BasisT {
   T m_inv[3], wagp[3], wegp[3], xegp[3];
   T mw[3][3];           // [mode][point] M_INV*WAGP
   T srfac[3][3];        // [mode][point] M_INV*WAGP*PHI_AREA (SRFAC without the area)
+  // The stage kernel's per-lane tables, copied to shared memory in this order:
+  // modes 2 and 3 at each edge point, and the edge weights as powers of two,
+  // EDGEQ(l, j, 2) = sw[..][0] * EDGEQ(1, 1, 1) and EDGEQ(l, j, 3) = sw[..][1],
+  // by side (ex: the points reversed; in) and the in side's point number
+  T tr[3][3][2];        // [led][point]
+  T sw[2][3][3][2];     // [in side][led][point]
 };
 using BasisP1 = BasisT<double>;
 static_assert(sizeof(BasisT<float>) * 2 == sizeof(BasisT<double>), "basis tables are plain arrays");
@@ -98,29 +105,32 @@ struct MeshView {
   const double* __restrict__ ibcfsb;
   const double* __restrict__ ibcfsp;
   // stage tile plan (built at create from the edge graph, rebuilt when the
-  // tile shape changes)
-  int max_halo, max_tasks;                // largest halo / task list of a tile
-  const int* __restrict__ tile_elem_ptr;  // [ntile+1] first element of each tile
-  const int* __restrict__ tile_task_ptr;  // [ntile+1] offsets into tile_tasks
-  const uint2* __restrict__ tile_tasks;   // TaskBits word, list index
-  const int* __restrict__ tile_halo_ptr;  // [ntile+1] offsets into tile_halo
-  const int* __restrict__ tile_halo;      // global element ids, ascending
+  // tile shape changes): tile t holds elements t * tile .. (the last one up to
+  // ne_tiled) and its tasks and halo at fixed strides, so that a block's first
+  // loads need no offsets
+  int ne_tiled;
+  int max_halo, max_tasks;                // largest halo / task list of a tile: the strides
+  const int2* __restrict__ tile_count;    // tasks of a tile, those of them (the first) that read no halo element
+  const uint2* __restrict__ tile_tasks;   // [tile][max_tasks] TaskBits word, list index
+  const int* __restrict__ tile_halo;      // [tile][max_halo] global element ids, ascending, then -1
   const unsigned* __restrict__ eslot;     // task of local edge l: bits 10l..10l+9
+  const void* __restrict__ tile_nrm;      // per task: normal from its in to its ex side (x, y), arithmetic type
 };
 
 // Stage tile shapes the stage kernel is compiled in: a tile of up to `tile`
-// consecutive elements and `threads` edge tasks per block of `threads`.
-// Every shape gives the same results bit for bit (each edge point's flux is
-// evaluated in the reference's in/ex orientation whichever tile evaluates
-// it, and each element's sums keep the reference's order); the autotuner
-// (dgswem_cuda_autotune) picks the fastest for a mesh.  `tile` is a multiple
-// of 32 (phase 3 keeps an area point per warp) and `threads` a multiple of
-// `tile` above it (phase 1 copies rows by whole groups of `tile` threads).
+// consecutive elements, whose at most `threads` = 3 or 4 x `tile` edge tasks
+// and `tile` elements a block of `block` threads works through.  Every shape
+// gives the same results bit for bit (each edge point's flux is evaluated in
+// the reference's in/ex orientation whichever tile evaluates it, and each
+// element's sums keep the reference's order); the autotuner
+// (dgswem_cuda_autotune) picks the fastest for a mesh.  `tile` is a multiple of
+// 32 and `block` a multiple of `tile` (phase 1 copies rows by whole groups of
+// `tile` threads).
 struct TileShape {
-  int tile, threads;
+  int tile, threads, block;
 };
 constexpr int kNumTileShapes = 4;
-constexpr TileShape kTileShapes[kNumTileShapes] = {{128, 384}, {64, 192}, {64, 256}, {256, 768}};
+constexpr TileShape kTileShapes[kNumTileShapes] = {{128, 384, 128}, {64, 192, 64}, {64, 256, 128}, {256, 768, 256}};
 constexpr int kDefaultTileShape = 0;
 // Block sizes of the limiter / WETDRY element kernel (limit_wetdry), each
 // compiled for 1024 resident threads per SM except the last (768: more
@@ -157,14 +167,12 @@ struct EGeo {
   static constexpr int kSmemRows = 14;
 };
 
-// Dynamic shared memory of the stage kernel (byte offsets).  Per-element
-// rows of geo: the first EGeo::kSmemRows rows of the table, then the hybrid
-// friction factor.
+// The p=2 kernel's shared geometry rows: the first EGeo::kSmemRows rows of the
+// table, then the hybrid friction factor.
 struct SGeo {
   static constexpr int kHyb = EGeo::kSmemRows;
 };
-constexpr int kGeoRows = EGeo::kSmemRows + 1;
-constexpr int kVolRows = 8;  // per area point: fx fy gx gy hx hy sx sy
+constexpr int kGeoRows = EGeo::kSmemRows + 1;  // of the p=2 kernel
 // doubles per element slot of the shared state: 12 modal values and a pad,
 // a 112-byte stride that keeps 16-byte loads by 8 consecutive slots free of
 // bank conflicts
@@ -173,8 +181,9 @@ constexpr unsigned kQStride = 14;
 // precision): the 12 modal values, three 16-byte loads, a 48-byte stride
 // that is conflict-free for 8 consecutive slots
 constexpr unsigned kQfStride = 12;
+// Dynamic shared memory of the stage kernel (byte offsets)
 struct StageLayout {
-  unsigned qs, geo, qf, vol, res, wd, gid, tdry, info, tasks, bytes;
+  unsigned qs, geo, qf, res, tab, wd, tflag, rare, bytes;
 };
 __host__ __device__ inline unsigned align16(unsigned x) { return (x + 15u) & ~15u; }
 // tile: elements per tile of the shape; rb: bytes of the arithmetic type of
@@ -185,22 +194,19 @@ __host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int 
   const unsigned nt = (unsigned)tile;
   const unsigned S = nt + (unsigned)max_halo;
   const unsigned T = (unsigned)max_tasks;
-  L.qs = 0;  // the basis tables are read from constant memory
+  L.qs = 0;
   // qs[S][kQStride]: ZE, QX, QY, HB modes (mixed: the tile's own slots only,
   // for the FP64 SSP combination; the edge and volume terms read qf)
-  L.geo = L.qs + kQStride * (rb == 8u ? S : nt) * 8u;
-  L.qf = L.geo + kGeoRows * nt * rb;           // geo[kGeoRows][tile] in the arithmetic type
-  L.vol = L.qf + (rb == 8u ? 0u : kQfStride * S * 4u);  // qf[S][kQfStride] (mixed only)
-  L.res = L.vol + kVolRows * 3u * nt * rb;     // vol[kVolRows][3][tile]
-  // res[task][point][5]; the mixed variant first stages the halo's FP64
-  // values there (12 doubles an element)
-  const unsigned res_bytes = 15u * T * rb, stage_bytes = rb == 8u ? 0u : 96u * (unsigned)max_halo;
-  L.wd = L.res + (res_bytes > stage_bytes ? res_bytes : stage_bytes);
-  L.gid = align16(L.wd + S * 4u);              // wd[S]
-  L.tdry = align16(L.gid + (unsigned)max_halo * 4u);
-  L.info = align16(L.tdry + T * 4u);          // einfo, eslot of the tile's elements
-  L.tasks = align16(L.info + 2u * nt * 4u);    // the tile's edge-task words (uint2)
-  L.bytes = align16(L.tasks + T * 8u);
+  const unsigned rows = L.qs + kQStride * (rb == 8u ? S : nt) * 8u;
+  // the geometry rows kDrdx .. kSmemRows-1 of the tile, row r at geo + r * tile
+  L.geo = rows - EGeo::kDrdx * nt * rb;
+  L.qf = rows + (EGeo::kSmemRows - EGeo::kDrdx) * nt * rb;  // qf[S][kQfStride] (mixed only)
+  L.res = L.qf + (rb == 8u ? 0u : kQfStride * S * 4u);      // res[task][point][F, G, H], an odd stride
+  L.tab = align16(L.res + 9u * T * rb);                     // BasisT::tr, sw
+  L.wd = align16(L.tab + 54u * rb);                         // wd[S]
+  L.tflag = align16(L.wd + S * 4u);                         // tflag[task]
+  L.rare = align16(L.tflag + T * 4u);                       // rare[1 + task]
+  L.bytes = align16(L.rare + (T + 1u) * 4u);
   return L;
 }
 
@@ -216,6 +222,10 @@ struct PhysF {
   float g, nleq, leq, nleqg, fg_l, tau_cap, cori, fric, cf;
 };
 
+// SSP-RK combinations of the p=1 stage kernel by their nonzero terms: any, the
+// first stage's ca q + cb rhs, and ca0 q(step start) + ca q + cb rhs
+enum SspKind { kSspAny = 0, kSspOne = 1, kSspTwo = 2 };
+
 struct StageArgs {
   MeshView m;
   Physics ph;
@@ -227,6 +237,8 @@ struct StageArgs {
   const double* rhist[kMaxStages];          // RHS of stage I<irk (if needed)
   double* rout;                             // this stage's RHS, or null
   double a[kMaxStages], b[kMaxStages];      // ATVD(irk,I), BTVD(irk,I)*DT
+  int ssp;                                  // SspKind
+  double ca0, ca, cb;
   const int* __restrict__ wd;               // WDFLG (read)
   double timedg, rampdg;
   const double* __restrict__ ramp;          // RAMPDG of this stage in device memory (graph replays), or null: rampdg
@@ -236,6 +248,8 @@ struct StageArgs {
   const double* __restrict__ wsy;
   const double* __restrict__ pr;
   double* ib_rhs;                           // [(2*seg + side)*9 + c] internal-barrier terms
+  double* xres;                             // [task][point][G, H] of the ex side of tasks with one dry side
+                                            // (in the arithmetic type)
   unsigned* err;                            // device error word
   // tiles of this launch: block b runs tile tile_list[tile_off + b], or
   // tile b when tile_list is null (all tiles)
@@ -264,6 +278,8 @@ struct LimitArgs {
   void set_basis(const BasisP1& b);                                                            \
   void launch_stage(const StageArgs& a, bool nonlin, int shape, unsigned grid, size_t smem,       \
                     cudaStream_t s);                                                           \
+  void launch_task_normals(const MeshView& m, int tile, void* out, unsigned ntile,             \
+                           cudaStream_t s);                                                    \
   void launch_ibarrier(const StageArgs& a, bool nonlin, cudaStream_t s);                       \
   void launch_node_minmax(const LimitArgs& a, unsigned grid, cudaStream_t s);                  \
   void launch_limit_wetdry(const LimitArgs& a, int shape, cudaStream_t s);                      \

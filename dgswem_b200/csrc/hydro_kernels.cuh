@@ -31,6 +31,8 @@ typedef double real;
 #endif
 __constant__ BasisT<real> cBasisR;  // cBasis in that type
 
+__device__ real gTab[54];  // BasisT::tr and sw, the stage kernel's per-lane tables
+
 // RAMPDG of the stage: from device memory in a replayed CUDA graph (whose
 // kernel arguments are fixed at capture), else the launch argument
 __device__ __forceinline__ double stage_ramp(const StageArgs& A) { return A.ramp ? *A.ramp : A.rampdg; }
@@ -98,6 +100,9 @@ template <class T>
 struct Flux3T {
   T f, g, h;
 };
+struct alignas(2 * sizeof(real)) Real2 {
+  real x, y;
+};
 using Flux3 = Flux3T<double>;
 
 // Total depth HT = ZE*NLEQ + HB of numerical_flux.F's flux evaluation.
@@ -106,20 +111,84 @@ __device__ __forceinline__ T depth(const Physics& P, T ze, T hb) {
   return kNonlin ? ze + hb : ze * T(P.nleq) + hb;
 }
 
+// max(|un| + c, |un|) with c the square root of a real number: |un| + c, or
+// |un| where c is NaN (a negative depth), since c >= 0 otherwise.  FP64 has no
+// maximum instruction: a select on c costs half of fmax's compare, selects
+// and NaN handling.  (c = NaN and |un| = NaN give NaN either way.)
+__device__ __forceinline__ double side_speed(double a, double c) { return c == c ? a + c : a; }
+__device__ __forceinline__ float side_speed(float a, float c) { return fmaxf(a + c, a); }
+
+// a b, never fused with a sum
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+// a b + c: fused in the contracting builds (not left to the compiler, which
+// may fuse another product of a sum of two), the product rounded by itself in
+// the strict build
+template <class T>
+__device__ __forceinline__ T madd(T a, T b, T c) {
+#ifdef DGSWEM_FAST_MATH
+  return fma(a, b, c);
+#else
+  return c + a * b;
+#endif
+}
+
+// 1 / d and sqrt(s) of both sides of an edge point (d = total depth, s =
+// gravity wave speed squared), FP64, by cr_math.cuh's sequences where all four
+// are in their range.  kTry: without a branch, ok reset where they are not --
+// the stage kernel forms an edge's three points in one straight line, which
+// the compiler interleaves, and redoes the edge out of line in that rare case;
+// otherwise the operators take over here, out of line.
+__device__ __noinline__ double rcp_any(double x) { return 1.0 / x; }
+__device__ __noinline__ double quot_any(double a, double b) { return a / b; }
+__device__ __noinline__ double sqrt_any(double x) { return sqrt(x); }
+template <bool kTry>
+__device__ __forceinline__ void side_terms(double di, double de, double si, double se, double& fi, double& fe,
+                                           double& ci, double& ce, bool& ok) {
+  const bool in = mid_range(di) && mid_range(de) && mid_range(si) && mid_range(se);
+  if (kTry || __builtin_expect(in, 1)) {
+    fi = rcp_from(di, rcp_seed(di));
+    fe = rcp_from(de, rcp_seed(de));
+    ci = sqrt_from(si, rsqrt_seed(si));
+    ce = sqrt_from(se, rsqrt_seed(se));
+    ok = ok && in;
+  } else {
+    fi = rcp_any(di);
+    fe = rcp_any(de);
+    ci = sqrt_any(si);
+    ce = sqrt_any(se);
+  }
+}
+template <bool kTry>
+__device__ __forceinline__ void side_terms(float di, float de, float si, float se, float& fi, float& fe, float& ci,
+                                           float& ce, bool&) {
+  fi = 1.0f / di;
+  fe = 1.0f / de;
+  ci = sqrtf(si);
+  ce = sqrtf(se);
+}
+// fmax without the NaN handling of FP64's (no maximum instruction)
+__device__ __forceinline__ double larger(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
+
 // numerical_flux.F:750-914, Local Lax-Friedrichs, in arithmetic type T.
 // kNonlin specialises NLEQ=1, LEQ=0 (the products with 1 and sums with 0 it
 // removes are exact).  ht_in / ht_ex: the total depths, depth(ze, hb) --
 // passed in so that the mixed-precision kernels can supply them from FP32
 // depth traces rather than from an FP32 sum of elevation and bathymetry.
-template <bool kNonlin, class T>
-__device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T qx_in, T qx_ex, T qy_in,
-                                         T qy_ex, T hb_in, T hb_ex, T ht_in, T ht_ex, T sf_in, T sf_ex, T nx,
-                                         T ny, T G) {
+template <bool kNonlin, class T, bool kTry = false>
+__device__ __forceinline__ Flux3T<T> llf_ok(const Physics& P, T ze_in, T ze_ex, T qx_in, T qx_ex, T qy_in,
+                                            T qy_ex, T hb_in, T hb_ex, T ht_in, T ht_ex, T sf_in, T sf_ex, T nx,
+                                            T ny, T G, bool& ok) {
   const T NLEQ = kNonlin ? T(1) : T(P.nleq);
   const T LEQ = kNonlin ? T(0) : T(P.leq);
   const T nleqg = G * NLEQ;
   const T j1 = ze_ex - ze_in, j2 = qx_ex - qx_in, j3 = qy_ex - qy_in;
-  T f1, fx1i, fy1i, fh, ui, vi, fx2i, fy2i, fx3i, fy3i;
+  const T nxsi = nx * sf_in, nxse = nx * sf_ex;
+  T fh, fhe, ci, ce;
+  side_terms<kTry>(kNonlin ? ht_in : NLEQ * ht_in + LEQ, kNonlin ? ht_ex : NLEQ * ht_ex + LEQ,
+                   G * ht_in * madd(nxsi, nxsi, mul_rn(ny, ny)), G * ht_ex * madd(nxse, nxse, mul_rn(ny, ny)), fh, fhe, ci, ce, ok);
+  T f1, fx1i, fy1i, ui, vi, fx2i, fy2i, fx3i, fy3i;
   {
     f1 = kNonlin ? T(1) : NLEQ + LEQ * hb_in;
     fx1i = qx_in * f1 * sf_in;
@@ -127,7 +196,6 @@ __device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T q
     const T fu = kNonlin ? qx_in : NLEQ * qx_in;
     const T fv = kNonlin ? qy_in : NLEQ * qy_in;
     const T fg = nleqg * ze_in;
-    fh = T(1) / (kNonlin ? ht_in : NLEQ * ht_in + LEQ);
     ui = qx_in * fh;
     vi = qy_in * fh;
     const T huu = fu * ui, hvv = fv * vi, huv = fu * vi;
@@ -145,7 +213,6 @@ __device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T q
     const T fu = kNonlin ? qx_ex : NLEQ * qx_ex;
     const T fv = kNonlin ? qy_ex : NLEQ * qy_ex;
     const T fg = nleqg * ze_ex;
-    const T fhe = T(1) / (kNonlin ? ht_ex : NLEQ * ht_ex + LEQ);
     ue = qx_ex * fhe;
     ve = qy_ex * fhe;
     const T huu = fu * ue, hvv = fv * ve, huv = fu * ve;
@@ -159,16 +226,12 @@ __device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T q
   const T f2a = T(0.5) * ((fx2i + fx2e) * nx + (fy2i + fy2e) * ny);
   const T f3a = T(0.5) * ((fx3i + fx3e) * nx + (fy3i + fy3e) * ny);
   const T uni = kNonlin ? ui * nx + vi * ny : (ui * nx + vi * ny) * NLEQ;
-  const T nxsi = nx * sf_in, nxse = nx * sf_ex;
-  const T ci = sqrt(G * ht_in * (ny * ny + nxsi * nxsi));
   const T une = kNonlin ? ue * nx + ve * ny : (ue * nx + ve * ny) * NLEQ;
-  const T ce = sqrt(G * ht_ex * (ny * ny + nxse * nxse));
   // max(|un+c|, |un|, |un-c|) over both sides.  For c >= 0 the rounded
   // |un| + c equals the rounded larger of |un + c| and |un - c| exactly, so
   // fmax(|un| + c, |un|) is the same value; with c = NaN (negative depth) both
   // forms reduce to |un|, as fmax skips NaN operands.
-  const T ai = fabs(uni), ae = fabs(une);
-  const T eig = fmax(fmax(ai + ci, ai), fmax(ae + ce, ae));
+  const T eig = larger(side_speed(fabs(uni), ci), side_speed(fabs(une), ce));
   Flux3T<T> r;
   r.f = f1a - T(0.5) * eig * j1;
   if (kNonlin) {
@@ -182,11 +245,12 @@ __device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T q
   return r;
 }
 
-__device__ __forceinline__ void load_basis(BasisP1& s) {
-  const double* src = reinterpret_cast<const double*>(&cBasis);
-  double* dst = reinterpret_cast<double*>(&s);
-  for (int i = threadIdx.x; i < (int)(sizeof(BasisP1) / sizeof(double)); i += blockDim.x) dst[i] = src[i];
-  __syncthreads();
+template <bool kNonlin, class T>
+__device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T qx_in, T qx_ex, T qy_in, T qy_ex,
+                                         T hb_in, T hb_ex, T ht_in, T ht_ex, T sf_in, T sf_ex, T nx, T ny, T G) {
+  bool ok;
+  return llf_ok<kNonlin, T>(P, ze_in, ze_ex, qx_in, qx_ex, qy_in, qy_ex, hb_in, hb_ex, ht_in, ht_ex, sf_in, sf_ex,
+                            nx, ny, G, ok);
 }
 
 // Trace of the modal state at point j of local edge l (mode 1 is 1 there).
@@ -379,29 +443,38 @@ __global__ void __launch_bounds__(128) ibarrier_sides(const __grid_constant__ St
 // up to kTile consecutive elements (the shape's tile), and for them the edge
 // tasks the tile evaluates (boundary edges, edges to out-of-tile elements,
 // shared interior edges once) and the halo of out-of-tile neighbours those
-// tasks read.  Four phases separated by barriers, each spread over all
-// kStageThreads threads:
+// tasks read.  Three phases separated by barriers, kTile threads:
 //   1. tile and halo elements: modal state, bathymetry modes and wet/dry flag
-//      into shared memory; tile elements also their geometry;
-//   2. one thread per (element, area point): volume fluxes and sources (tile
-//      elements only: in the FP64 variants the halo's copies are still in
-//      flight, waited for at the end of this phase);
-//   3. one thread per (task, Lobatto point): the LLF flux of an edge point in
-//      the reference's own in/ex orientation with its dry-side rules ->
-//      F, G_in, H_in, G_ex, H_ex (internal-barrier sides come from
-//      ibarrier_sides);
-//   4. one thread per (element, mode): that mode of the three variables
-//      summed in the reference's order (boundary edges, interior edges in
-//      edge-number order as the slot sum of add_internal_flux, rain, area
-//      points), then the SSP combination.
+//      into shared memory; tile elements also the geometry rows the sums read;
+//   2. one thread per edge task: its two elements' modes once into registers,
+//      then the LLF flux at the three Lobatto points in the reference's own
+//      in/ex orientation with its dry-side rules -> F, G, H per point in
+//      shared memory (internal-barrier sides come from ibarrier_sides);
+//   3. one thread per element: the nine right-hand sides, each in the
+//      reference's order (boundary edges, interior edges in edge-number order
+//      as the slot sum of add_internal_flux, rain, area points), the volume
+//      fluxes and sources formed where they are added, then the SSP
+//      combination.
+// Work is split by edge and by element, not by point and mode, because the
+// kernel is bound by instruction issue: a finer split repeats the loads of an
+// element's modes, the task decode, the weights and the geometry for every
+// point and mode (4,670 thread instructions an element and stage in the first
+// stage, 1,550 of them FP64, against 2,270 and 1,180 here), and because the
+// values of one edge or element give straight-line code whose long dependent
+// chains (reciprocals, roots) the compiler interleaves: with a branch per
+// operation, as the operators' range checks make, a block of the kernel took
+// twice the cycles.  Three blocks of 128 threads with 168 registers and no
+// spills: four blocks of 128 registers, five of 96 and six of 80 spill and are
+// 11, 25 and 40 % slower.  On 1M elements (strict, wet/dry beach, mean of the
+// two stages) 245 us before, 144 us now.
 // internal_edge_hydro.F, *_edge_hydro.F, rhs_dg_hydro.F, DG_hydro_timestep.F:238-290
 // ---------------------------------------------------------------------------
 
-// resident stage threads per SM the register allocation targets (FP64: two
-// blocks of 384, at most 85 registers a thread); a shape of T threads per
-// block is compiled for that many over T resident blocks
+// resident stage threads per SM the register allocation targets (FP64: 128
+// registers a thread); a shape of T threads per block is compiled for that
+// many over T resident blocks
 #ifndef DGSWEM_STAGE_RESIDENT_THREADS
-#define DGSWEM_STAGE_RESIDENT_THREADS 768
+#define DGSWEM_STAGE_RESIDENT_THREADS 384
 #endif
 constexpr int stage_min_blocks(int threads) {
   return DGSWEM_STAGE_RESIDENT_THREADS / threads > 0 ? DGSWEM_STAGE_RESIDENT_THREADS / threads : 1;
@@ -428,17 +501,17 @@ __device__ __forceinline__ void slot_values(const real* qt, int slot, real v[12]
 #endif
 }
 
-// Trace at edge point (led, gp) of slot `slot`'s ZE, QX, QY and HB; mode 0
-// of the basis is 1 on every edge point.
-__device__ __forceinline__ void slot_trace(const BasisT<real>& B, const real* qt, int slot, int led, int gp,
-                                           real& z, real& u, real& v, real& h) {
-  const real p1 = B.phi_edge[led][gp][1], p2 = B.phi_edge[led][gp][2];
-  real q[12];
-  slot_values(qt, slot, q);
-  z = q[0] + q[1] * p1 + q[2] * p2;
-  u = q[3] + q[4] * p1 + q[5] * p2;
-  v = q[6] + q[7] * p1 + q[8] * p2;
-  h = q[9] + q[10] * p1 + q[11] * p2;
+// q0 + q1 p1 + q2 p2, a trace at Lobatto point I from a variable's three
+// modes.  At the end points (vertices) p1 and p2 are 0, +-1 or 2
+// (BasisT::tr): the products are exact and the fused form gives the bits of
+// the separately rounded one.  At the midpoint they are +-1/2 (or -1 and 0),
+// exact except for subnormal modes, which waves running into still water do
+// reach: there the strict build rounds the products.
+__device__ __forceinline__ real trace3(int I, const real* q, real p1, real p2) {
+#ifndef DGSWEM_FAST_MATH
+  if (I == 1) return q[0] + q[1] * p1 + q[2] * p2;
+#endif
+  return fma(q[2], p2, fma(q[1], p1, q[0]));
 }
 
 // One Lobatto point of an interior edge in the reference's in/ex orientation
@@ -505,274 +578,467 @@ __device__ __forceinline__ void trace_depth(const Physics& P, real z, real w, re
 #endif
 }
 
-// Volume fluxes and sources at area point I of element e (rhs_dg_hydro.F:
-// 58-470) from the element's 12 slot values q (ZE, QX, QY modes, then HB or,
-// in the mixed variant, depth modes), its inverse Jacobian, element-mean
-// Manning n and hybrid friction factor: out = fx fy gx gy hx hy sx sy.
-template <bool kNonlin, bool kSph>
-__device__ __forceinline__ void volume_core(const StageArgs& A, const BasisT<real>& C, const real q[12], real drdx,
-                                            real dsdx, real drdy, real dsdy, real nbar, real hyb, int I, int e,
-                                            real out[8]) {
+// The volume terms' reciprocal, square root and Manning friction G n^2 /
+// depth^(1/3): FP64 by cr_math.cuh's sequences without a branch, ok reset where
+// an argument is out of their range (a zero speed is in it), and by the
+// operators, out of line, for those.
+__device__ __forceinline__ double rcp_try(double x, bool& ok) {
+  ok = ok && mid_range(x);
+  return rcp_from(x, rcp_seed(x));
+}
+__device__ __forceinline__ double sqrt_try(double x, bool& ok) {
+  ok = ok && (mid_range(x) || x == 0.0);
+  const double r = sqrt_from(x, rsqrt_seed(x));
+  return x == 0.0 ? x : r;
+}
+__device__ __forceinline__ double manning_try(double gn2, double depth, bool& ok) {
+#ifdef DGSWEM_FAST_MATH
+  return gn2 / cbrt(depth);
+#else
+  double c;
+  const bool near = pow_third_try(depth, &c);
+  ok = ok && near && mid_range(gn2) && mid_range(c);
+  return quot_from(gn2, c, rcp_from(c, rcp_seed(c)));
+#endif
+}
+__device__ __forceinline__ double rcp_slow(double x) { return rcp_any(x); }
+__device__ __forceinline__ double sqrt_slow(double x) { return sqrt_any(x); }
+__device__ __forceinline__ double manning_slow(double gn2, double depth) { return quot_any(gn2, cube_root(depth)); }
+__device__ __forceinline__ float rcp_try(float x, bool&) { return 1.0f / x; }
+__device__ __forceinline__ float sqrt_try(float x, bool&) { return sqrtf(x); }
+__device__ __forceinline__ float manning_try(float gn2, float depth, bool&) { return gn2 / cube_root(depth); }
+__device__ __forceinline__ float rcp_slow(float x) { return 1.0f / x; }
+__device__ __forceinline__ float sqrt_slow(float x) { return sqrtf(x); }
+__device__ __forceinline__ float manning_slow(float gn2, float depth) { return gn2 / cube_root(depth); }
+
+// Adds the volume integral of element e (rhs_dg_hydro.F:58-470) to its nine
+// right-hand sides from its 12 slot values q (ZE, QX, QY modes, then HB or, in
+// the mixed variant, depth modes) and geometry rows.  What is the same at the
+// three area points is formed once: the mode derivatives' products with the
+// inverse Jacobian (drphi and dsphi are constants at p=1: modes 2 and 3 have
+// d/dx = 3/2 dsdx and drdx + 1/2 dsdx), the bed slope, M_INV * WAGP, the
+// vertices' wind stress and pressure scaled by the ramp (met_forcing.F:49-66).
+// The three points' reciprocals, square roots and cube roots come first and in
+// straight lines -- long dependent chains, which the compiler interleaves --
+// with one test that they are all in range at the end (ok).
+template <bool kNonlin, bool kSph, int kTile>
+__device__ __forceinline__ void volume_sums(const StageArgs& A, const BasisT<real>& C, const real q[12],
+                                            const real* geo, int el, int e, real rhs[3][3]) {
   const MeshView& m = A.m;
   const Physics& P = A.ph;
   const PhysR R = phys_r(A);
   const int ne = m.ne;
-  const int wde = 1;  // volume terms are evaluated for wet elements only
+  const real NLEQ = kNonlin ? real(1) : R.nleq, LEQ = kNonlin ? real(0) : R.leq;
 #ifdef DGSWEM_MIXED
-  // the slot holds the depth modes ZE + HB (see trace_depth)
-  const real hbe[3] = {q[9] - q[0], q[10] - q[1], q[11] - q[2]};
+  const real hbe[3] = {q[9] - q[0], q[10] - q[1], q[11] - q[2]};  // the slot holds the depth modes ZE + HB
 #else
   const real* hbe = q + 9;
 #endif
-  const real NLEQ = kNonlin ? real(1) : R.nleq, LEQ = kNonlin ? real(0) : R.leq;
-  const real cori = m.cori ? (real)m.cori[e] : R.cori;
-  real fric = m.fric ? (real)m.fric[e] : R.fric;
-  real zq = q[0], uq = q[3], vq = q[6];
-  const real hq = hbe[0] * C.phi_area[0][I] + hbe[1] * C.phi_area[1][I] + hbe[2] * C.phi_area[2][I];
-  real dhx = 0, dhy = 0;
+  real zq[3], uq[3], vq[3], hq[3], depth[3], fh[3], tau[3];
+  bool ok = true;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    dhx = dhx + hbe[k] * (C.drphi[k][I] * drdx + C.dsphi[k][I] * dsdx);
-    dhy = dhy + hbe[k] * (C.drphi[k][I] * drdy + C.dsphi[k][I] * dsdy);
-  }
-  zq = zq + q[1] * C.phi_area[1][I] + q[2] * C.phi_area[2][I];
-  uq = uq + q[4] * C.phi_area[1][I] + q[5] * C.phi_area[2][I];
-  vq = vq + q[7] * C.phi_area[1][I] + q[8] * C.phi_area[2][I];
+  for (int I = 0; I < 3; ++I) {
+    hq[I] = hbe[0] * C.phi_area[0][I] + hbe[1] * C.phi_area[1][I] + hbe[2] * C.phi_area[2][I];
+    zq[I] = q[0] + q[1] * C.phi_area[1][I] + q[2] * C.phi_area[2][I];
+    uq[I] = q[3] + q[4] * C.phi_area[1][I] + q[5] * C.phi_area[2][I];
+    vq[I] = q[6] + q[7] * C.phi_area[1][I] + q[8] * C.phi_area[2][I];
 #ifdef DGSWEM_MIXED
-  const real depth =
-      kNonlin ? q[9] + q[10] * C.phi_area[1][I] + q[11] * C.phi_area[2][I] : zq + hq;
+    depth[I] = kNonlin ? q[9] + q[10] * C.phi_area[1][I] + q[11] * C.phi_area[2][I] : zq[I] + hq[I];
 #else
-  const real depth = zq + hq;
+    depth[I] = zq[I] + hq[I];
 #endif
-  const real sfq = kSph ? (real)m.sfac_area[(size_t)I * ne + e] : real(1);
-  const real f1 = kNonlin ? real(1) : NLEQ + LEQ * hq;
-  const real fx = uq * f1 * sfq, fy = vq * f1;
-  const real fu = kNonlin ? uq : NLEQ * uq, fv = kNonlin ? vq : NLEQ * vq;
-  const real fg = R.nleqg * zq * wde;
-  const real fh = real(1) / (kNonlin ? depth : NLEQ * depth + LEQ);
-  const real u = uq * fh, v = vq * fh;
-  const real huu = fu * u, hvv = fv * v, huv = fu * v;
-  const real gh2 = kNonlin ? fg * (real(0.5) * zq + hq) : fg * (real(0.5) * zq + hq) + R.fg_l * zq;
-  const real gx = (huu + gh2) * sfq, gy = huv;
-  const real hx = huv * sfq, hy = hvv + gh2;
+    fh[I] = rcp_try(kNonlin ? depth[I] : NLEQ * depth[I] + LEQ, ok);
+    tau[I] = m.fric ? (real)m.fric[e] : R.fric;
+  }
+  real gn2 = 0;
   if (m.manning) {
-    fric = R.g * (nbar * nbar) / cube_root(depth);
-    if (fric < R.cf) fric = R.cf;
-  }
-  real tau = fric;
-  if (P.iflinbf == 0) {
-    const real umag = sqrt(u * u + v * v);
-    tau = tau * umag * fh;
-    if (P.ifhybf == 1) tau = tau * hyb;
-    tau = fmin(tau, R.tau_cap);
-  }
-  real sx = -(tau * uq) + fg * dhx * sfq + cori * vq;
-  real sy = -(tau * vq) + fg * dhy - cori * uq;
-  if (P.nws != 0) {
-    // met_forcing.F:49-66: the nodal fields are scaled by the ramp each stage
-    const real drpsi[3] = {-0.5, 0.5, 0.0}, dspsi[3] = {-0.5, 0.0, 0.5};
-    real dpsidx[3], dpsidy[3];
+    const real nbar = geo[EGeo::kNbar * kTile + el];
+    gn2 = R.g * (nbar * nbar);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      dpsidx[a] = drpsi[a] * drdx + dspsi[a] * dsdx;
-      dpsidy[a] = drpsi[a] * drdy + dspsi[a] * dsdy;
+    for (int I = 0; I < 3; ++I) {
+      tau[I] = manning_try(gn2, depth[I], ok);
+      tau[I] = tau[I] < R.cf ? R.cf : tau[I];
     }
-    const real fw = real(1) / f1, r = (real)stage_ramp(A);
-    const int n0 = m.nm[e], n1 = m.nm[(size_t)ne + e], n2 = m.nm[(size_t)2 * ne + e];
-    const real wx0 = r * (real)A.wsx[n0], wx1 = r * (real)A.wsx[n1], wx2 = r * (real)A.wsx[n2];
-    const real wy0 = r * (real)A.wsy[n0], wy1 = r * (real)A.wsy[n1], wy2 = r * (real)A.wsy[n2];
-    const real p0 = r * (real)A.pr[n0], p1 = r * (real)A.pr[n1], p2 = r * (real)A.pr[n2];
-    sx = sx + fw * (wx0 * C.psi[0][I] + wx1 * C.psi[1][I] + wx2 * C.psi[2][I]) -
-         R.g * sfq * depth * (p0 * dpsidx[0] + p1 * dpsidx[1] + p2 * dpsidx[2]);
-    sy = sy + fw * (wy0 * C.psi[0][I] + wy1 * C.psi[1][I] + wy2 * C.psi[2][I]) -
-         R.g * depth * (p0 * dpsidy[0] + p1 * dpsidy[1] + p2 * dpsidy[2]);
   }
-  out[0] = fx; out[1] = fy; out[2] = gx; out[3] = gy;
-  out[4] = hx; out[5] = hy; out[6] = sx; out[7] = sy;
-}
-
-// Phase 3 of the stage kernel for area point I of tile element el (global
-// id e): volume_core on the element's shared-memory slot and geometry rows,
-// into vol[(v*3 + I)*kTile + el] by volume_point.  C: the basis tables in
-// shared memory (I is a runtime index); qt: the slots in the arithmetic type.
-template <bool kNonlin, bool kSph, int kTile>
-__device__ __forceinline__ void volume_values(const StageArgs& A, const BasisT<real>& C, const real* qt,
-                                              const real* geo, int I, int el, int e, real out[8]) {
-  real q[12];
-  slot_values(qt, el, q);
+  if (P.iflinbf == 0) {
+#pragma unroll
+    for (int I = 0; I < 3; ++I) {
+      const real u = uq[I] * fh[I], v = vq[I] * fh[I];
+      tau[I] = tau[I] * sqrt_try(u * u + v * v, ok) * fh[I];
+    }
+  }
+  if (__builtin_expect(!ok, 0)) {
+#pragma unroll 1
+    for (int I = 0; I < 3; ++I) {
+      const real d = I == 0 ? depth[0] : I == 1 ? depth[1] : depth[2];
+      const real f = rcp_slow(kNonlin ? d : NLEQ * d + LEQ);
+      real t = m.fric ? (real)m.fric[e] : R.fric;
+      if (m.manning) {
+        t = manning_slow(gn2, d);
+        if (t < R.cf) t = R.cf;
+      }
+      if (P.iflinbf == 0) {
+        const real u = (I == 0 ? uq[0] : I == 1 ? uq[1] : uq[2]) * f;
+        const real v = (I == 0 ? vq[0] : I == 1 ? vq[1] : vq[2]) * f;
+        t = t * sqrt_slow(u * u + v * v) * f;
+      }
+#pragma unroll
+      for (int J = 0; J < 3; ++J)
+        if (I == J) { fh[J] = f; tau[J] = t; }
+    }
+  }
+  if (P.iflinbf == 0) {
+    real hyb = 1;
+    if (P.ifhybf == 1) {  // hybrid friction factor from the element-mean depth
+#ifdef DGSWEM_MIXED
+      const real depth_c = q[9];
+#else
+      const real depth_c = q[9] + q[0];
+#endif
+      const real fh_c = real(1) / (kNonlin ? depth_c : real(P.nleq) * depth_c + real(P.leq));
+      hyb = pow(real(1) + pow(real(P.hbreak) * fh_c, real(P.ftheta)), real(P.fgamma / P.ftheta));
+    }
+#pragma unroll
+    for (int I = 0; I < 3; ++I) {
+      if (P.ifhybf == 1) tau[I] = tau[I] * hyb;
+      tau[I] = tau[I] < R.tau_cap ? tau[I] : R.tau_cap;
+    }
+  }
   const real drdx = geo[EGeo::kDrdx * kTile + el], dsdx = geo[EGeo::kDsdx * kTile + el];
   const real drdy = geo[EGeo::kDrdy * kTile + el], dsdy = geo[EGeo::kDsdy * kTile + el];
-  const real nbar = A.m.manning ? geo[EGeo::kNbar * kTile + el] : real(0);
-  const real hyb = (A.ph.iflinbf == 0 && A.ph.ifhybf == 1) ? geo[SGeo::kHyb * kTile + el] : real(0);
-  volume_core<kNonlin, kSph>(A, C, q, drdx, dsdx, drdy, dsdy, nbar, hyb, I, e, out);
-}
-
-template <bool kNonlin, bool kSph, int kTile>
-__device__ __forceinline__ void volume_point(const StageArgs& A, const BasisT<real>& C, const real* qt,
-                                             const real* geo, real* vol, int I, int el, int e) {
-  real v[8];
-  volume_values<kNonlin, kSph, kTile>(A, C, qt, geo, I, el, e, v);
+  const real x1 = real(1.5) * dsdx, x2 = drdx + real(0.5) * dsdx;
+  const real y1 = real(1.5) * dsdy, y2 = drdy + real(0.5) * dsdy;
+  const real dhx = madd(hbe[2], x2, hbe[1] * x1), dhy = madd(hbe[2], y2, hbe[1] * y1);
+  const real xf1 = C.mw[1][0] * x1, yf1 = C.mw[1][0] * y1, xf2 = C.mw[2][0] * x2, yf2 = C.mw[2][0] * y2;
+  const real cori = m.cori ? (real)m.cori[e] : R.cori;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) vol[(r * 3 + I) * kTile + el] = v[r];
+  for (int I = 0; I < 3; ++I) {
+    const real sfq = kSph ? (real)m.sfac_area[(size_t)I * ne + e] : real(1);
+    const real f1 = kNonlin ? real(1) : NLEQ + LEQ * hq[I];
+    const real fx = uq[I] * f1 * sfq, fy = vq[I] * f1;
+    const real fu = kNonlin ? uq[I] : NLEQ * uq[I], fv = kNonlin ? vq[I] : NLEQ * vq[I];
+    const real fg = R.nleqg * zq[I];
+    const real u = uq[I] * fh[I], v = vq[I] * fh[I];
+    const real huu = fu * u, hvv = fv * v, huv = fu * v;
+    const real gt = real(0.5) * zq[I] + hq[I];
+    const real gh2 = kNonlin ? real(0) : fg * gt + R.fg_l * zq[I];
+    const real gx = (kNonlin ? madd(fg, gt, huu) : huu + gh2) * sfq, gy = huv;
+    const real hx = huv * sfq, hy = kNonlin ? madd(fg, gt, hvv) : hvv + gh2;
+    real sx = -(tau[I] * uq[I]) + fg * dhx * sfq + cori * vq[I];
+    real sy = -(tau[I] * vq[I]) + fg * dhy - cori * uq[I];
+    if (P.nws != 0) {
+      // met_forcing.F:49-66: the nodal fields are scaled by the ramp each stage
+      const real drpsi[3] = {-0.5, 0.5, 0.0}, dspsi[3] = {-0.5, 0.0, 0.5};
+      real dpsidx[3], dpsidy[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        dpsidx[a] = drpsi[a] * drdx + dspsi[a] * dsdx;
+        dpsidy[a] = drpsi[a] * drdy + dspsi[a] * dsdy;
+      }
+      const real fw = real(1) / f1, r = (real)stage_ramp(A);
+      const int n0 = m.nm[e], n1 = m.nm[(size_t)ne + e], n2 = m.nm[(size_t)2 * ne + e];
+      const real wx0 = r * (real)A.wsx[n0], wx1 = r * (real)A.wsx[n1], wx2 = r * (real)A.wsx[n2];
+      const real wy0 = r * (real)A.wsy[n0], wy1 = r * (real)A.wsy[n1], wy2 = r * (real)A.wsy[n2];
+      const real p0 = r * (real)A.pr[n0], p1 = r * (real)A.pr[n1], p2 = r * (real)A.pr[n2];
+      sx = sx + fw * (wx0 * C.psi[0][I] + wx1 * C.psi[1][I] + wx2 * C.psi[2][I]) -
+           R.g * sfq * depth[I] * (p0 * dpsidx[0] + p1 * dpsidx[1] + p2 * dpsidx[2]);
+      sy = sy + fw * (wy0 * C.psi[0][I] + wy1 * C.psi[1][I] + wy2 * C.psi[2][I]) -
+           R.g * depth[I] * (p0 * dpsidy[0] + p1 * dpsidy[1] + p2 * dpsidy[2]);
+    }
+    const real s0 = C.srfac[0][I], s1 = C.srfac[1][I], s2 = C.srfac[2][I];
+    rhs[1][0] = rhs[1][0] + s0 * sx;
+    rhs[2][0] = rhs[2][0] + s0 * sy;
+    rhs[0][1] = rhs[0][1] + xf1 * fx + yf1 * fy;
+    rhs[1][1] = rhs[1][1] + xf1 * gx + yf1 * gy + s1 * sx;
+    rhs[2][1] = rhs[2][1] + xf1 * hx + yf1 * hy + s1 * sy;
+    rhs[0][2] = rhs[0][2] + xf2 * fx + yf2 * fy;
+    rhs[1][2] = rhs[1][2] + xf2 * gx + yf2 * gy + s2 * sx;
+    rhs[2][2] = rhs[2][2] + xf2 * hx + yf2 * hy + s2 * sy;
+  }
 }
 
-// Phase 4 of the stage kernel for mode K of tile element el (global id e):
-// the right-hand side of mode K of the three variables, each summed in the
-// reference's order -- boundary edges, interior edges in edge-number order
-// (the slot sum of add_internal_flux), rain, area points -- then the SSP
-// combination (DG_hydro_timestep.F:238-290) written to qout.  The edge and
-// area-point weights of mode K are formed once for the three variables.  The
-// basis tables come from constant memory (cBasisR): K is the same for a
-// whole warp and the point indices are fixed by unrolled loops; the edge
-// weights' per-lane (edge, point) rows cost a few distinct addresses a warp
-// but keep the load off the shared-memory pipe.  The sums are in the arithmetic
-// type, the SSP combination in FP64 (in the mixed variant: the RHS rounded
-// to FP32, the stage states and their combination FP64).
-template <bool kNonlin, int kTile>
-__device__ __forceinline__ void sum_mode(const StageArgs& A, const double* qs,
-                                         const real* geo, const real* vol, const real* res, const int* tdry,
-                                         const unsigned* sinfo, const int* wds, const uint2* stasks, int K, int el,
-                                         int e) {
+// Phase 2 of the stage kernel: an edge task of the tile (word tk, normal
+// (nx, ny) from the in to the ex side), its three Lobatto points.  o[3*point +
+// {0, 1, 2}] = F, G, H of the in side, and of the ex side unless one of the two
+// is dry: then xres holds the ex side's G and H, xo[2*point + {0, 1}].  tflag: 0, kTaskDry where both sides are dry (no flux), or
+// kTaskTwo where one is (the dry-side rules of internal_edge_hydro.F:212-302).
+constexpr int kTaskDry = 1, kTaskTwo = 2;
+
+// Lobatto point I of a task the main path leaves out: an interior task with one
+// dry side or with a value outside the range of llf_ok's sequences, or a
+// boundary task.
+template <bool kNonlin, bool kSph, int kTile>
+__device__ __forceinline__ void edge_point_rare(const StageArgs& A, const real* tab, const real* qt, const int* wds,
+                                                int tile0, int hbeg, uint2 tk, Real2 nrm, int I, real* o, real* xo) {
+  const MeshView& m = A.m;
+  const Physics& P = A.ph;
+  const int ne = m.ne;
+  const unsigned fl = tk.x, kind = fl & 7u;
+  const int sin = (fl >> TaskBits::kInSlot) & 511, led_in = (fl >> TaskBits::kLedIn) & 3;
+  const real nx = nrm.x, ny = nrm.y;
+  const real* ti = tab + led_in * 6;
+  real q[12];
+  slot_values(qt, sin, q);
+  const real pi1 = ti[2 * I], pi2 = ti[2 * I + 1];
+  const real zi = trace3(I, q, pi1, pi2), xi = trace3(I, q + 3, pi1, pi2), yi = trace3(I, q + 6, pi1, pi2);
+  real hi, hti, f[5];
+  trace_depth<kNonlin>(P, zi, trace3(I, q + 9, pi1, pi2), hi, hti);
+  const int gin = kSph ? (sin < kTile ? tile0 + sin : m.tile_halo[hbeg + sin - kTile]) : 0;
+  const real sfi = kSph ? (real)m.sfac_edge[(size_t)(led_in * 3 + I) * ne + gin] : real(1);
+  if (kind == kInterior) {
+    const int sex = (fl >> TaskBits::kExSlot) & 511, led_ex = (fl >> TaskBits::kLedEx) & 3;
+    const real* tx = tab + led_ex * 6 + 4;
+    const real px1 = tx[-2 * I], px2 = tx[-2 * I + 1];
+    slot_values(qt, sex, q);
+    const real zx = trace3(I, q, px1, px2), xx = trace3(I, q + 3, px1, px2), yx = trace3(I, q + 6, px1, px2);
+    real hx, htx;
+    trace_depth<kNonlin>(P, zx, trace3(I, q + 9, px1, px2), hx, htx);
+    const int gex = kSph ? (sex < kTile ? tile0 + sex : m.tile_halo[hbeg + sex - kTile]) : 0;
+    const real sfx = kSph ? (real)m.sfac_edge[(size_t)(led_ex * 3 + 2 - I) * ne + gex] : real(1);
+    interior_point<kNonlin>(P, zi, zx, xi, xx, yi, yx, hi, hx, hti, htx, sfi, sfx, nx, ny, wds[sin], wds[sex], f);
+    xo[2 * I] = f[3];
+    xo[2 * I + 1] = f[4];
+  } else {
+    real zx, xx, yx;
+    ghost_state(A, kind, (int)tk.y, I, zi, xi, yi, hi, nx, ny, zx, xx, yx);
+    // only the ocean ghost has its own elevation (the others copy zi)
+    const real htx = kind == kOcean ? depth<kNonlin>(P, zx, hi) : hti;
+    const Flux3T<real> r =
+        llf<kNonlin, real>(P, zi, zx, xi, xx, yi, yx, hi, hi, hti, htx, sfi, sfi, nx, ny, real(P.g));
+    f[0] = r.f; f[1] = r.g; f[2] = r.h;
+  }
+  o[3 * I] = f[0];
+  o[3 * I + 1] = f[1];
+  o[3 * I + 2] = f[2];
+}
+
+// Returns whether the task is left to edge_point_rare.
+template <bool kNonlin, bool kSph, int kTile>
+__device__ __forceinline__ bool edge_task(const StageArgs& A, const real* tab, const real* qt, const int* wds,
+                                          int tile0, int hbeg, uint2 tk, real nx, real ny, real* o, int* flag) {
+  const MeshView& m = A.m;
+  const Physics& P = A.ph;
+  const int ne = m.ne;
+  const unsigned fl = tk.x, kind = fl & 7u;
+  const int sin = (fl >> TaskBits::kInSlot) & 511;
+  const int wd_in = wds[sin];
+  // (barrier sides: ibarrier_sides, launched before this kernel)
+  if (kind != kInterior) return kind != kIBarrier && wd_in != 0;
+  const int sex = (fl >> TaskBits::kExSlot) & 511;
+  const int wd_ex = wds[sex];
+  const bool both = wd_in != 0 && wd_ex != 0, none = wd_in == 0 && wd_ex == 0;
+  *flag = both ? 0 : none ? kTaskDry : kTaskTwo;
+  if (!both) return !none;
+  const int led_in = (fl >> TaskBits::kLedIn) & 3, led_ex = (fl >> TaskBits::kLedEx) & 3;
+  const real* ti = tab + led_in * 6;
+  const real* tx = tab + led_ex * 6 + 4;  // the ex side's points run backwards
+  const int gin = kSph ? (sin < kTile ? tile0 + sin : m.tile_halo[hbeg + sin - kTile]) : 0;
+  const int gex = kSph ? (sex < kTile ? tile0 + sex : m.tile_halo[hbeg + sex - kTile]) : 0;
+  real qi[12], qx[12];
+  slot_values(qt, sin, qi);
+  slot_values(qt, sex, qx);
+  bool ok = true;
+#pragma unroll
+  for (int I = 0; I < 3; ++I) {
+    const real pi1 = ti[2 * I], pi2 = ti[2 * I + 1], px1 = tx[-2 * I], px2 = tx[-2 * I + 1];
+    const real zi = trace3(I, qi, pi1, pi2), xi = trace3(I, qi + 3, pi1, pi2), yi = trace3(I, qi + 6, pi1, pi2);
+    const real zx = trace3(I, qx, px1, px2), xx = trace3(I, qx + 3, px1, px2), yx = trace3(I, qx + 6, px1, px2);
+    real hi, hti, hx, htx;
+    trace_depth<kNonlin>(P, zi, trace3(I, qi + 9, pi1, pi2), hi, hti);
+    trace_depth<kNonlin>(P, zx, trace3(I, qx + 9, px1, px2), hx, htx);
+    const real sfi = kSph ? (real)m.sfac_edge[(size_t)(led_in * 3 + I) * ne + gin] : real(1);
+    const real sfx = kSph ? (real)m.sfac_edge[(size_t)(led_ex * 3 + 2 - I) * ne + gex] : real(1);
+    const Flux3T<real> f = llf_ok<kNonlin, real, true>(P, zi, zx, xi, xx, yi, yx, hi, hx, hti, htx, sfi, sfx, nx, ny,
+                                                       real(P.g), ok);
+    o[3 * I] = f.f;
+    o[3 * I + 1] = f.g;
+    o[3 * I + 2] = f.h;
+  }
+  return !ok;
+}
+
+// Phase 3 of the stage kernel: tile element el (global id e).
+// The sums are in the arithmetic type, the SSP combination in FP64 (in the
+// mixed variant: the RHS rounded to FP32, the stage states and their
+// combination FP64).
+template <bool kNonlin, bool kSph, int kTile>
+__device__ __forceinline__ void element_sums(const StageArgs& A, const real* tab, const double* qs, const real* qt,
+                                             const real* geo, const real* res, const int* tflag, const int* wds,
+                                             int tbeg, unsigned info, unsigned slots, int el, int e) {
   const BasisT<real>& C = cBasisR;
   const MeshView& m = A.m;
   const Physics& P = A.ph;
   const int ne = m.ne;
-  // SSP terms of stage 1 fetched first so that their latency overlaps the
-  // sums below; the combination keeps the reference's order
-  const bool hist0 = A.irk > 1;
-  double h0q[3] = {0.0, 0.0, 0.0}, h0r[3] = {0.0, 0.0, 0.0};
-  if (hist0) {
-#pragma unroll
-    for (int V = 0; V < 3; ++V) {
-      const size_t c = (size_t)(3 * V + K) * ne + e;
-      if (A.a[0] != 0.0) h0q[V] = A.qhist[0][c];
-      if (A.b[0] != 0.0) h0r[V] = A.rhist[0][c];
-    }
-  }
-  const unsigned info = sinfo[el], slots = sinfo[kTile + el];
   const int wde = wds[el];
-  real rhs[3] = {0, 0, 0}, isum[3] = {0, 0, 0};
+  real rhs[3][3], isum[3][3];  // [variable][mode]
 #pragma unroll
-  for (int s = 0; s < 3; ++s) {
-    const int l = ei_order(info, s);
-    const unsigned kind = ei_kind(info, l);
-    if (kind == kNone) continue;
-    const int ti = (slots >> (10 * l)) & kNoTask;
-    const real* r = res + (size_t)ti * 15;
-    if (kind == kIBarrier) {
-      const double* o = A.ib_rhs + (size_t)stasks[ti].y * 9;
+  for (int V = 0; V < 3; ++V)
 #pragma unroll
-      for (int V = 0; V < 3; ++V) rhs[V] = rhs[V] + (real)o[3 * V + K];
-      continue;
-    }
-    if (kind == kInterior) {
-      if (tdry[ti]) continue;
-      const bool is_in = ei_flag(info, l) != 0;
-      const int c1 = is_in ? 1 : 3;  // G and H of this side: components c1, c1 + 1
-      const real edfac = geo[(EGeo::kEdfac + l) * kTile + el];
-      real acc[3] = {0, 0, 0};
+    for (int K = 0; K < 3; ++K) { rhs[V][K] = 0; isum[V][K] = 0; }
+  // one interior edge l in the order of the sum, its flux at r: the nine
+  // weights EDFAC * EDGEQ(l, point, mode), negative on the in side
+  // (rhs_*_in(k) - w_in * flux), are powers of two times two numbers: EDGEQ is
+  // 1/3 (rounded) times 1, 4, 1 for mode 1 and times the factors sw[..][0] for
+  // mode 2, and is itself the power of two sw[..][1] for mode 3 (BasisT::sw,
+  // checked when the tables are built).
+  auto add_edge = [&](int l, const real v[3][3]) {
+    const bool is_in = ei_flag(info, l) != 0;
+    const real ed = geo[(EGeo::kEdfac + l) * kTile + el];
+    const real a = ed * C.edgeq[0][0][0];
+    const real wa = is_in ? -a : a, we = is_in ? -ed : ed;
+    const real* sw = tab + 18 + (is_in ? 18 : 0) + l * 6;
+    real acc[3][3];
 #pragma unroll
-      for (int I = 0; I < 3; ++I) {
-        const int j = is_in ? I : 2 - I;
-        const real wk = edfac * C.edgeq[l][j][K];  // constant memory: off the shared-memory pipe
-        const real* rv = r + 5 * I;
-        const real val[3] = {rv[0], rv[c1], rv[c1 + 1]};
+    for (int I = 0; I < 3; ++I) {
+      const real w[3] = {I == 1 ? real(4) * wa : wa, sw[2 * I] * wa, sw[2 * I + 1] * we};
 #pragma unroll
-        for (int V = 0; V < 3; ++V) {
-          if (is_in)  // rhs_*_in(k) = rhs_*_in(k) - w_in * flux
-            acc[V] = acc[V] - wk * val[V];
-          else        // rhs_*_ex(k) = rhs_*_ex(k) + w_ex * flux
-            acc[V] = acc[V] + wk * val[V];
+      for (int V = 0; V < 3; ++V)
+#pragma unroll
+        for (int K = 0; K < 3; ++K) {
+          acc[V][K] = I == 0 ? mul_rn(w[K], v[I][V]) : madd(w[K], v[I][V], acc[V][K]);
         }
+    }
+#pragma unroll
+    for (int V = 0; V < 3; ++V)
+#pragma unroll
+      for (int K = 0; K < 3; ++K) isum[V][K] = isum[V][K] + acc[V][K];
+  };
+  bool plain = (info & 0x1ffu) == 0u;  // three interior edges (kInterior is 0), none with a dry side
+  static_assert(kInterior == 0, "einfo's kind bits");
+#pragma unroll
+  for (int l = 0; l < 3; ++l) plain = plain && tflag[plain ? (slots >> (10 * l)) & kNoTask : 0] == 0;
+  if (__builtin_expect(plain, 1)) {
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const int l = ei_order(info, s);
+      const real* r = res + ((slots >> (10 * l)) & kNoTask) * 9;
+      real v[3][3];
+#pragma unroll
+      for (int I = 0; I < 3; ++I)
+#pragma unroll
+        for (int V = 0; V < 3; ++V) v[I][V] = r[3 * I + V];
+      add_edge(l, v);
+    }
+  } else {
+#pragma unroll 1
+    for (int s = 0; s < 3; ++s) {
+      const int l = ei_order(info, s);
+      const unsigned kind = ei_kind(info, l);
+      if (kind == kNone) continue;
+      const int ti = (slots >> (10 * l)) & kNoTask;
+      const real* r = res + ti * 9;
+      if (kind == kIBarrier) {
+        const double* o = A.ib_rhs + (size_t)m.tile_tasks[tbeg + ti].y * 9;
+#pragma unroll
+        for (int V = 0; V < 3; ++V)
+#pragma unroll
+          for (int K = 0; K < 3; ++K) rhs[V][K] = rhs[V][K] + (real)o[3 * V + K];
+        continue;
       }
+      if (kind == kInterior) {
+        const int tf = tflag[ti];
+        if (tf == kTaskDry) continue;
+        real v[3][3];  // [point][F, G, H]
 #pragma unroll
-      for (int V = 0; V < 3; ++V) isum[V] = isum[V] + acc[V];
-    } else {
-      if (wde == 0) continue;
-      const real areas = egeo_r(m)[(size_t)EGeo::kAreas * ne + e];
-      const real xlen = egeo_r(m)[(size_t)(EGeo::kXlen + l) * ne + e];
+        for (int I = 0; I < 3; ++I)
 #pragma unroll
-      for (int I = 0; I < 3; ++I) {
-        const real wk = real(2) * C.m_inv[K] / areas * xlen * C.phi_edge[l][I][K] * C.wegp[I];
+          for (int V = 0; V < 3; ++V) v[I][V] = r[3 * I + V];
+        if (tf == kTaskTwo && ei_flag(info, l) == 0) {
+          const real* xr = reinterpret_cast<const real*>(A.xres) + (size_t)(tbeg + ti) * 6;
 #pragma unroll
-        for (int V = 0; V < 3; ++V) rhs[V] = rhs[V] - wk * r[5 * I + V];
+          for (int I = 0; I < 3; ++I) { v[I][1] = xr[2 * I]; v[I][2] = xr[2 * I + 1]; }
+        }
+        add_edge(l, v);
+      } else if (wde != 0) {
+        const real areas = egeo_r(m)[(size_t)EGeo::kAreas * ne + e];
+        const real xlen = egeo_r(m)[(size_t)(EGeo::kXlen + l) * ne + e];
+        const real wb[3] = {real(2) * C.m_inv[0] / areas * xlen, real(2) * C.m_inv[1] / areas * xlen,
+                            real(2) * C.m_inv[2] / areas * xlen};
+#pragma unroll
+        for (int I = 0; I < 3; ++I)
+#pragma unroll
+          for (int K = 0; K < 3; ++K) {
+            const real wk = wb[K] * C.phi_edge[l][I][K] * C.wegp[I];
+#pragma unroll
+            for (int V = 0; V < 3; ++V) rhs[V][K] = rhs[V][K] - wk * r[3 * I + V];
+          }
       }
     }
   }
 #pragma unroll
-  for (int V = 0; V < 3; ++V) rhs[V] = rhs[V] + isum[V];  // add_internal_flux
+  for (int V = 0; V < 3; ++V)
+#pragma unroll
+    for (int K = 0; K < 3; ++K) rhs[V][K] = rhs[V][K] + isum[V][K];  // add_internal_flux
   if (P.rainfall == 1) {
     const real src = real(7.0556e-6);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) rhs[0] = rhs[0] + C.srfac[K][i] * src;
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int K = 0; K < 3; ++K) rhs[0][K] = rhs[0][K] + C.srfac[K][i] * src;
   }
+  // the step-start state of the SSP combination, in one batch here: its latency
+  // is covered by the volume terms (read where it is used, between stores that
+  // the compiler cannot reorder, nine round trips cost 70 us of 260 at 1M
+  // elements; after the volume terms 3 us; prefetched before the edge sums 3 us)
+  double h0[9];
+  if (A.ssp == kSspTwo)
+#pragma unroll
+    for (int c = 0; c < 9; ++c) h0[c] = A.qhist[0][(size_t)c * ne + e];
   if (wde != 0) {
-    const real drdx = geo[EGeo::kDrdx * kTile + el], dsdx = geo[EGeo::kDsdx * kTile + el];
-    const real drdy = geo[EGeo::kDrdy * kTile + el], dsdy = geo[EGeo::kDsdy * kTile + el];
-    // vol rows: fx fy gx gy hx hy sx sy, each [point][tile]
+    real q[12];
+    slot_values(qt, el, q);
+    volume_sums<kNonlin, kSph, kTile>(A, C, q, geo, el, e, rhs);
+  }
+  // SSP-RK combination (DG_hydro_timestep.F:238-290), zero coefficients
+  // skipped: the stages whose nonzero terms are the current state and
+  // right-hand side (the first), or those and the step-start state, without a
+  // branch per term
+  bool bad = false;
+  double out[9];
+  if (A.ssp != kSspAny) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const real sr = C.srfac[K][i];
-      const real sx = vol[(6 * 3 + i) * kTile + el], sy = vol[(7 * 3 + i) * kTile + el];
-      if (K == 0) {
-        rhs[1] = rhs[1] + sr * sx;
-        rhs[2] = rhs[2] + sr * sy;
-      } else {
-        const real dpx = C.drphi[K][i] * drdx + C.dsphi[K][i] * dsdx;
-        const real dpy = C.drphi[K][i] * drdy + C.dsphi[K][i] * dsdy;
-        const real xf = C.mw[K][i] * dpx;
-        const real yf = C.mw[K][i] * dpy;
-        const real fx = vol[(0 * 3 + i) * kTile + el], fy = vol[(1 * 3 + i) * kTile + el];
-        const real gx = vol[(2 * 3 + i) * kTile + el], gy = vol[(3 * 3 + i) * kTile + el];
-        const real hx = vol[(4 * 3 + i) * kTile + el], hy = vol[(5 * 3 + i) * kTile + el];
-        rhs[0] = rhs[0] + xf * fx + yf * fy;
-        rhs[1] = rhs[1] + xf * gx + yf * gy + sr * sx;
-        rhs[2] = rhs[2] + xf * hx + yf * hy + sr * sy;
+    for (int c = 0; c < 9; ++c) {
+      double acc = 0.0;
+      if (A.ssp == kSspTwo) acc = madd(A.ca0, h0[c], acc);
+      acc = madd(A.ca, qs[el * kQStride + c], acc);
+      out[c] = madd(A.cb, (double)rhs[c / 3][c % 3], acc);
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+      double acc = 0.0;
+      for (int I = 0; I < A.irk; ++I) {
+        const bool cur = I == A.irk - 1;
+        if (A.a[I] != 0.0) acc = acc + A.a[I] * (cur ? qs[el * kQStride + c] : A.qhist[I][(size_t)c * ne + e]);
+        if (A.b[I] != 0.0) acc = acc + A.b[I] * (cur ? (double)rhs[c / 3][c % 3] : A.rhist[I][(size_t)c * ne + e]);
       }
+      out[c] = acc;
     }
   }
-  // SSP-RK combination (DG_hydro_timestep.F:238-290); zero coefficients skipped
-  bool bad = false;
 #pragma unroll
-  for (int V = 0; V < 3; ++V) {
-    const int c = 3 * V + K;
-    const double rk = (double)rhs[V];
-    if (A.rout) A.rout[(size_t)c * ne + e] = rk;
-    const double qc = qs[el * kQStride + c];
-    double acc = 0.0;
-    if (hist0) {
-      if (A.a[0] != 0.0) acc = acc + A.a[0] * h0q[V];
-      if (A.b[0] != 0.0) acc = acc + A.b[0] * h0r[V];
-    }
-    for (int I = 1; I < A.irk; ++I) {
-      const bool cur = I == A.irk - 1;
-      if (A.a[I] != 0.0) acc = acc + A.a[I] * (cur ? qc : A.qhist[I][(size_t)c * ne + e]);
-      if (A.b[I] != 0.0) acc = acc + A.b[I] * (cur ? rk : A.rhist[I][(size_t)c * ne + e]);
-    }
-    if (!hist0) {  // stage 1: the current stage is I = 0
-      if (A.a[0] != 0.0) acc = acc + A.a[0] * qc;
-      if (A.b[0] != 0.0) acc = acc + A.b[0] * rk;
-    }
-    bad = bad || isnan(acc);
-    A.qout[(size_t)c * ne + e] = acc;
+  for (int c = 0; c < 9; ++c) {
+    bad = bad || isnan(out[c]);
+    A.qout[(size_t)c * ne + e] = out[c];
+  }
+  if (A.rout) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) A.rout[(size_t)c * ne + e] = (double)rhs[c / 3][c % 3];
   }
   if (bad) atomicOr(A.err, 1u);
 }
 
-template <bool kNonlin, bool kSph, int kTile, int kStageThreads>
-__global__ void __launch_bounds__(kStageThreads, stage_min_blocks(kStageThreads))
+template <bool kNonlin, bool kSph, int kTile, int kThreads>
+__global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
     stage_p1(const __grid_constant__ StageArgs A) {
-  static_assert(kTile % 32 == 0 && kStageThreads % kTile == 0 && kStageThreads > kTile, "tile shape");
+  static_assert(kTile % 32 == 0 && kThreads % kTile == 0, "tile shape");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const MeshView& m = A.m;
-  const Physics& P = A.ph;
   const int ne = m.ne;
   const int tid = threadIdx.x;
   const int tile = A.tile_list ? A.tile_list[A.tile_off + (int)blockIdx.x] : (int)blockIdx.x;
-  const int tile0 = m.tile_elem_ptr[tile];
-  const int n = m.tile_elem_ptr[tile + 1] - tile0;
-  const int hbeg = m.tile_halo_ptr[tile], nh = m.tile_halo_ptr[tile + 1] - hbeg;
-  const int tbeg = m.tile_task_ptr[tile], ntask = m.tile_task_ptr[tile + 1] - tbeg;
+  const int tile0 = tile * kTile, n = min(kTile, m.ne_tiled - tile0);
+  const int hbeg = tile * m.max_halo, tbeg = tile * m.max_tasks;
+  const int2 count = m.tile_count[tile];  // tasks, those of them that read no halo element
   const StageLayout L = stage_layout(kTile, m.max_halo, m.max_tasks, (unsigned)sizeof(real));
   double* qs = reinterpret_cast<double*>(smem_raw + L.qs);
   real* geo = reinterpret_cast<real*>(smem_raw + L.geo);
@@ -781,244 +1047,154 @@ __global__ void __launch_bounds__(kStageThreads, stage_min_blocks(kStageThreads)
 #else
   const real* qt = qs;
 #endif
-  real* vol = reinterpret_cast<real*>(smem_raw + L.vol);
   real* res = reinterpret_cast<real*>(smem_raw + L.res);
+  real* tab = reinterpret_cast<real*>(smem_raw + L.tab);  // BasisT::tr, then BasisT::sw
   int* wds = reinterpret_cast<int*>(smem_raw + L.wd);
-  int* gid = reinterpret_cast<int*>(smem_raw + L.gid);
-  int* tdry = reinterpret_cast<int*>(smem_raw + L.tdry);
-  unsigned* sinfo = reinterpret_cast<unsigned*>(smem_raw + L.info);  // [einfo | eslot][kTile]
-  uint2* stasks = reinterpret_cast<uint2*>(smem_raw + L.tasks);      // the tile's edge-task words
+  int* tflag = reinterpret_cast<int*>(smem_raw + L.tflag);
+  int* rare = reinterpret_cast<int*>(smem_raw + L.rare);  // number, then ids, of the tasks left to edge_point_rare
 
   // ---- phase 1: tile and halo elements into shared memory ----
-#ifdef DGSWEM_MIXED
-  // Thread w < kTile: tile element w's 12 modal values (state rows and
-  // bathymetry rows; consecutive threads on consecutive elements of a row)
-  // into registers, then its FP32 slot and the FP64 state the SSP
-  // combination reads.  The other threads: the geometry rows and flags
-  // (cp.async) and the halo elements' FP32 slots, one thread per element.
-  {
-    static_assert(kStageThreads > kTile && (kStageThreads - kTile) % kTile == 0,
-                  "geometry rows are copied by whole groups of kTile threads");
-    if (tid < kTile) {
-      if (tid < n) {
-        double v[12];
-        const double* src = A.qin + tile0 + tid;
-#pragma unroll
-        for (int r = 0; r < 9; ++r) v[r] = src[(size_t)r * ne];
-        src = m.hb + tile0 + tid;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) v[9 + k] = src[(size_t)k * ne];
-        double2* d = reinterpret_cast<double2*>(qs + tid * kQStride);
-#pragma unroll
-        for (int j = 0; j < 5; ++j) d[j] = make_double2(v[2 * j], v[2 * j + 1]);
-        // FP32 slot: ZE, QX, QY modes and the depth modes ZE + HB (FP64 sums)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) v[9 + k] = v[k] + v[9 + k];
-        float4* f = reinterpret_cast<float4*>(qt + tid * kQfStride);
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          f[j] = make_float4((float)v[4 * j], (float)v[4 * j + 1], (float)v[4 * j + 2], (float)v[4 * j + 3]);
-        // hybrid friction factor from the element-mean depth (depth mode 1)
-        if (P.iflinbf == 0 && P.ifhybf == 1) {
-          const real depth_c = (real)v[9];
-          const real fh_c = real(1) / (kNonlin ? depth_c : real(P.nleq) * depth_c + real(P.leq));
-          geo[SGeo::kHyb * kTile + tid] =
-              pow(real(1) + pow(real(P.hbreak) * fh_c, real(P.ftheta)), real(P.fgamma / P.ftheta));
-        }
-      }
-    } else {
-      constexpr int kU = kStageThreads - kTile, kStep = kU / kTile;
-      const int u = tid - kTile, w = u % kTile, r0 = u / kTile;
-      if (w < n) {
-        const int ngeo = m.manning ? EGeo::kSmemRows : EGeo::kNbar;
-        const size_t step = (size_t)kStep * ne;
-        const unsigned gdst = smem_addr(geo) + (unsigned)(r0 * kTile + w) * 4u;
-        const real* gsrc = egeo_r(m) + (size_t)r0 * ne + tile0 + w;
-#pragma unroll
-        for (int j = 0; j < (EGeo::kSmemRows + kStep - 1) / kStep; ++j)
-          if (r0 + j * kStep < ngeo) cp_async4_s(gdst + 4u * kStep * kTile * j, gsrc + j * step);
-#pragma unroll
-        for (int j = 0; j < (3 + kStep - 1) / kStep; ++j) {
-          const int r = r0 + j * kStep;
-          if (r == 0)
-            cp_async4(wds + w, A.wd + tile0 + w);
-          else if (r < 3)
-            cp_async4(sinfo + (r - 1) * kTile + w, (r == 1 ? m.einfo : m.eslot) + tile0 + w);
-        }
-      }
-      for (int j = u; j < ntask; j += kU) cp_async8(stasks + j, m.tile_tasks + tbeg + j);
-      cp_async_commit();
-      // halo element j: its 12 FP64 values staged by cp.async in the flux
-      // region (unused until the edge phase) and converted to its FP32 slot
-      // after the volume phase, so that the gather overlaps that phase
-      const unsigned hst = smem_addr(res);
-      for (int j = u; j < nh; j += kU) {
-        const int g = m.tile_halo[hbeg + j];
-        gid[j] = g;
-        cp_async4(wds + kTile + j, A.wd + g);
-#pragma unroll
-        for (int r = 0; r < 9; ++r) cp_async8_s(hst + 96u * j + 8u * r, A.qin + (size_t)r * ne + g);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) cp_async8_s(hst + 96u * j + 72u + 8u * k, m.hb + (size_t)k * ne + g);
-      }
-      cp_async_commit();
-    }
-    cp_async_wait_prior();
+  if (tid < 54) {  // from global memory: constant loads by lane would be replayed 32 times
+    if (sizeof(real) == 8)
+      cp_async8(tab + tid, gTab + tid);
+    else
+      cp_async4(tab + tid, gTab + tid);
   }
-  __syncthreads();
-#else
-  // Asynchronous global->shared copies (cp.async), no register staging, in
-  // two groups: the tile's rows (state, bathymetry, geometry table, flags;
-  // consecutive threads on consecutive elements of a row) and task words,
-  // then the halo elements (thread j: halo element j's 13 values).  The
-  // volume phase needs only the first group; the halo lands meanwhile.
-  const int hg = tid < nh ? m.tile_halo[hbeg + tid] : -1;
+  // Everything whose address is known: this thread's first task and its
+  // element's edge info into registers, the tile's rows by cp.async, and the
+  // halo ids, whose elements are copied once they and the tile are here.  The
+  // first round of edge tasks reads only tile elements: the halo's second round
+  // trip hides behind it.  (A block of more threads than tile elements, for
+  // meshes of few tiles, lets the others fetch the halo meanwhile and has one
+  // round of tasks.)
+  uint2 tk = make_uint2(kIBarrier, 0u);
+  Real2 nrm{};
+  if (tid < m.max_tasks) {
+    tk = m.tile_tasks[tbeg + tid];
+    nrm = reinterpret_cast<const Real2*>(m.tile_nrm)[tbeg + tid];
+  }
+  if (tid == 0) rare[0] = 0;
+  const int hj = kThreads > kTile ? tid - kTile : tid;
+  const int hid = hj >= 0 && hj < m.max_halo ? m.tile_halo[hbeg + hj] : -1;
+  unsigned info = 0, slots = 0;
+  if (tid < n) {
+    info = m.einfo[tile0 + tid];
+    slots = m.eslot[tile0 + tid];
+  }
   {
-    // thread t: element t % kTile of every (kStageThreads / kTile)-th row;
-    // shared addresses as 32-bit offsets, rows unrolled
-    static_assert(kStageThreads % kTile == 0, "tile rows are copied by whole groups of kTile threads");
-    constexpr int kRowStep = kStageThreads / kTile;
+    constexpr int kStep = kThreads / kTile;  // thread t: element t % kTile of every kStep-th row
     const int w = tid % kTile, r0 = tid / kTile;
-    const unsigned qs_s = smem_addr(qs), geo_s = smem_addr(geo);
     if (w < n) {
-      const int ngeo = m.manning ? EGeo::kSmemRows : EGeo::kNbar;
-      const size_t step = (size_t)kRowStep * ne;
-      const unsigned qdst = qs_s + (unsigned)(w * kQStride + r0) * 8u;
-      const double* src = A.qin + (size_t)r0 * ne + tile0 + w;
-#pragma unroll
-      for (int j = 0; j < (9 + kRowStep - 1) / kRowStep; ++j)
-        if (r0 + j * kRowStep < 9) cp_async8_s(qdst + 8u * kRowStep * j, src + j * step);
-      src = m.hb + (size_t)r0 * ne + tile0 + w;
-#pragma unroll
-      for (int j = 0; j < (3 + kRowStep - 1) / kRowStep; ++j)
-        if (r0 + j * kRowStep < 3) cp_async8_s(qdst + 72u + 8u * kRowStep * j, src + j * step);
+      const size_t step = (size_t)kStep * ne;
+      const int nrow = m.manning ? EGeo::kSmemRows : EGeo::kNbar;
       constexpr unsigned rb = sizeof(real);
-      const unsigned gdst = geo_s + (unsigned)(r0 * kTile + w) * rb;
-      const real* gsrc = egeo_r(m) + (size_t)r0 * ne + tile0 + w;
+      const unsigned gdst = smem_addr(geo) + (unsigned)((EGeo::kDrdx + r0) * kTile + w) * rb;
+      const real* gsrc = egeo_r(m) + (size_t)(EGeo::kDrdx + r0) * ne + tile0 + w;
 #pragma unroll
-      for (int j = 0; j < (EGeo::kSmemRows + kRowStep - 1) / kRowStep; ++j) {
-        if (r0 + j * kRowStep >= ngeo) continue;
+      for (int j = 0; j < (EGeo::kSmemRows - EGeo::kDrdx + kStep - 1) / kStep; ++j) {
+        if (EGeo::kDrdx + r0 + j * kStep >= nrow) continue;
         if (rb == 8)
-          cp_async8_s(gdst + rb * kRowStep * kTile * j, gsrc + j * step);
+          cp_async8_s(gdst + rb * kStep * kTile * j, gsrc + j * step);
         else
-          cp_async4_s(gdst + rb * kRowStep * kTile * j, gsrc + j * step);
+          cp_async4_s(gdst + rb * kStep * kTile * j, gsrc + j * step);
       }
-#pragma unroll
-      for (int j = 0; j < (3 + kRowStep - 1) / kRowStep; ++j) {
-        const int r = r0 + j * kRowStep;
-        if (r == 0)
-          cp_async4(wds + w, A.wd + tile0 + w);
-        else if (r < 3)
-          cp_async4(sinfo + (r - 1) * kTile + w, (r == 1 ? m.einfo : m.eslot) + tile0 + w);
-      }
+      if (r0 == 0) cp_async4(wds + w, A.wd + tile0 + w);
     }
-    for (int j = tid; j < ntask; j += kStageThreads) cp_async8(stasks + j, m.tile_tasks + tbeg + j);
-    cp_async_commit();
-    for (int j = tid; j < nh; j += kStageThreads) {
-      const int g = j == tid ? hg : m.tile_halo[hbeg + j];
-      gid[j] = g;
-      const unsigned hdst = qs_s + (unsigned)((kTile + j) * kQStride) * 8u;
-      const double* q0 = A.qin + g;
-#pragma unroll
-      for (int c = 0; c < 9; ++c) cp_async8_s(hdst + 8u * c, q0 + (size_t)c * ne);
-      const double* h0 = m.hb + g;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) cp_async8_s(hdst + 72u + 8u * k, h0 + (size_t)k * ne);
-      cp_async4(wds + kTile + j, A.wd + g);
-    }
-    cp_async_commit();
-    // hybrid friction factor of tile element tid from the element-mean depth
-    // (HB + ZE of mode 1, the operands the slot gets), for the volume phase
-    if (P.iflinbf == 0 && P.ifhybf == 1 && tid < n) {
-      const real depth_c = (real)(m.hb[tile0 + tid] + A.qin[tile0 + tid]);
-      const real fh_c = real(1) / (kNonlin ? depth_c : real(P.nleq) * depth_c + real(P.leq));
-      geo[SGeo::kHyb * kTile + tid] =
-          pow(real(1) + pow(real(P.hbreak) * fh_c, real(P.ftheta)), real(P.fgamma / P.ftheta));
-    }
-    cp_async_wait_prior();
   }
-  __syncthreads();
-#endif
-
-  // ---- phase 2: volume fluxes and sources per (element, area point) ----
-  // (the point is the same for a whole warp: kTile is a multiple of 32)
-  for (int w = tid; w < 3 * kTile; w += kStageThreads) {
-    const int i = w / kTile, el = w - i * kTile;
-    if (el >= n || wds[el] == 0) continue;
-    volume_point<kNonlin, kSph, kTile>(A, cBasisR, qt, geo, vol, i, el, tile0 + el);
-  }
-  cp_async_wait_all();  // the halo group
 #ifdef DGSWEM_MIXED
-  for (int j = tid - kTile; j >= 0 && j < nh; j += kStageThreads - kTile) {
-    const double* d = reinterpret_cast<const double*>(res) + 12 * j;  // this thread's staged copies
-    float v[12];
+  // one thread per tile or halo element: its 12 FP64 values into registers,
+  // then its FP32 slot (ZE, QX, QY modes and the depth modes ZE + HB, FP64
+  // sums) and, for a tile element, the FP64 state the SSP combination reads
+  auto load_slot = [&](int j, int g) {
+    double v[12];
 #pragma unroll
-    for (int r = 0; r < 9; ++r) v[r] = (float)d[r];
+    for (int r = 0; r < 9; ++r) v[r] = A.qin[(size_t)r * ne + g];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) v[9 + k] = (float)(d[k] + d[9 + k]);
-    float4* f = reinterpret_cast<float4*>(qt + (kTile + j) * kQfStride);
+    for (int k = 0; k < 3; ++k) v[9 + k] = m.hb[(size_t)k * ne + g];
+    if (j < kTile) {
+      double2* d = reinterpret_cast<double2*>(qs + j * kQStride);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) f[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-  }
-#endif
-  __syncthreads();
-
-  // ---- phase 3: one thread per (edge task, Lobatto point) ----
-  // (the three points of a task on adjacent lanes: same slots, broadcast loads)
-  for (int w = tid; w < 3 * ntask; w += kStageThreads) {
-    const int ti = w / 3, I = w - 3 * ti;
-    const uint2 tk = stasks[ti];
-    const unsigned fl = tk.x;
-    const unsigned kind = fl & 7u;
-    if (kind == kIBarrier) continue;  // ibarrier_sides, launched before this kernel
-    real* o = res + (size_t)ti * 15 + 5 * I;
-    const int sin = (fl >> TaskBits::kInSlot) & 511, sex = (fl >> TaskBits::kExSlot) & 511;
-    const int led_in = (fl >> TaskBits::kLedIn) & 3, led_ex = (fl >> TaskBits::kLedEx) & 3;
-    const bool flip = (fl >> TaskBits::kFlip) & 1u;
-    const int owner = flip ? sex : sin, oled = flip ? led_ex : led_in;
-    real nx = geo[(EGeo::kNx + oled) * kTile + owner], ny = geo[(EGeo::kNy + oled) * kTile + owner];
-    if (flip) { nx = -nx; ny = -ny; }
-    const int wd_in = wds[sin];
-    // global ids for the ics=2 tables
-    const int gin = sin < kTile ? tile0 + sin : gid[sin - kTile];
-    if (kind == kInterior) {
-      const int wd_ex = wds[sex];
-      const int dry = wd_in == 0 && wd_ex == 0;
-      if (I == 0) tdry[ti] = dry;
-      if (dry) continue;
-      const int gex = sex < kTile ? tile0 + sex : gid[sex - kTile];
-      const int gp_in = I, gp_ex = 2 - I;
-      real zi, xi, yi, wi, zx, xx, yx, wx, hi, hti, hx, htx;
-      slot_trace(cBasisR, qt, sin, led_in, gp_in, zi, xi, yi, wi);
-      slot_trace(cBasisR, qt, sex, led_ex, gp_ex, zx, xx, yx, wx);
-      trace_depth<kNonlin>(P, zi, wi, hi, hti);
-      trace_depth<kNonlin>(P, zx, wx, hx, htx);
-      const real sfi = kSph ? (real)m.sfac_edge[(size_t)(led_in * 3 + gp_in) * ne + gin] : real(1);
-      const real sfx = kSph ? (real)m.sfac_edge[(size_t)(led_ex * 3 + gp_ex) * ne + gex] : real(1);
-      interior_point<kNonlin>(P, zi, zx, xi, xx, yi, yx, hi, hx, hti, htx, sfi, sfx, nx, ny, wd_in, wd_ex, o);
+      for (int i = 0; i < 5; ++i) d[i] = make_double2(v[2 * i], v[2 * i + 1]);
     } else {
-      if (wd_in == 0) continue;
-      real zi, xi, yi, wi, zx, xx, yx, hi, hti;
-      slot_trace(cBasisR, qt, sin, led_in, I, zi, xi, yi, wi);
-      trace_depth<kNonlin>(P, zi, wi, hi, hti);
-      const real sfi = kSph ? (real)m.sfac_edge[(size_t)(led_in * 3 + I) * ne + gin] : real(1);
-      ghost_state(A, kind, (int)tk.y, I, zi, xi, yi, hi, nx, ny, zx, xx, yx);
-      // only the ocean ghost has its own elevation (the others copy zi)
-      const real htx = kind == kOcean ? depth<kNonlin>(P, zx, hi) : hti;
-      const Flux3T<real> f =
-          llf<kNonlin, real>(P, zi, zx, xi, xx, yi, yx, hi, hi, hti, htx, sfi, sfi, nx, ny, real(P.g));
-      o[0] = f.f; o[1] = f.g; o[2] = f.h;
+      wds[j] = A.wd[g];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[9 + k] = v[k] + v[9 + k];
+    float4* f = reinterpret_cast<float4*>(qt + j * kQfStride);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      f[i] = make_float4((float)v[4 * i], (float)v[4 * i + 1], (float)v[4 * i + 2], (float)v[4 * i + 3]);
+  };
+#else
+  auto load_slot = [&](int j, int g) {
+    const unsigned d = smem_addr(qs) + (unsigned)(j * kQStride) * 8u;
+    const double* q0 = A.qin + g;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) cp_async8_s(d + 8u * c, q0 + (size_t)c * ne);
+    const double* h0 = m.hb + g;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) cp_async8_s(d + 72u + 8u * k, h0 + (size_t)k * ne);
+    if (j >= kTile) cp_async4(wds + j, A.wd + g);
+  };
+#endif
+  bool halo_here = kThreads > kTile;
+  if (kThreads > kTile) {  // the threads beyond the tile's copy the halo
+    if (tid < kTile) {
+      if (tid < n) load_slot(tid, tile0 + tid);
+    } else {
+      for (int j = tid - kTile; j < m.max_halo; j += kThreads - kTile) {
+        const int g = j == tid - kTile ? hid : m.tile_halo[hbeg + j];
+        if (g >= 0) load_slot(kTile + j, g);
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+  } else {
+    if (tid < n) load_slot(tid, tile0 + tid);
+    cp_async_wait_all();
+    __syncthreads();
+    for (int j = tid; j < m.max_halo; j += kThreads) {
+      const int g = j == tid ? hid : m.tile_halo[hbeg + j];
+      if (g >= 0) load_slot(kTile + j, g);
     }
   }
-  __syncthreads();
 
-
-  // ---- phase 4: per (element, mode) sums in the reference's order, SSP ----
-  for (int w = tid; w < 3 * kTile; w += kStageThreads) {
-    const int K = w / kTile, el = w - K * kTile;
-    if (el >= n) continue;
-    sum_mode<kNonlin, kTile>(A, qs, geo, vol, res, tdry, sinfo, wds, stasks, K, el, tile0 + el);
+  // ---- phase 2: one thread per edge task (the next round's task is fetched
+  // while this one's is evaluated) ----
+  for (int t0 = 0; t0 < count.x; t0 += kThreads) {
+    if (!halo_here && t0 + kThreads > count.y) {
+      cp_async_wait_all();
+      __syncthreads();
+      halo_here = true;
+    }
+    const int t = t0 + tid;
+    const uint2 tk0 = tk;
+    const Real2 n0 = nrm;
+    if (t + kThreads < count.x) {
+      tk = m.tile_tasks[tbeg + t + kThreads];
+      nrm = reinterpret_cast<const Real2*>(m.tile_nrm)[tbeg + t + kThreads];
+    }
+    if (t < count.x &&
+        edge_task<kNonlin, kSph, kTile>(A, tab, qt, wds, tile0, hbeg, tk0, n0.x, n0.y, res + t * 9, tflag + t))
+      rare[1 + atomicAdd(rare, 1)] = t;
   }
+  __syncthreads();
+  // the tasks left out, a thread per (task, point): in any order, each writes
+  // its own values
+  const int nrare = rare[0];
+  if (nrare > 0) {
+    for (int w = tid; w < 3 * nrare; w += kThreads) {
+      const int i = w / 3, t = rare[1 + i];
+      edge_point_rare<kNonlin, kSph, kTile>(A, tab, qt, wds, tile0, hbeg, m.tile_tasks[tbeg + t],
+                                            reinterpret_cast<const Real2*>(m.tile_nrm)[tbeg + t], w - 3 * i,
+                                            res + t * 9, reinterpret_cast<real*>(A.xres) + (size_t)(tbeg + t) * 6);
+    }
+    __syncthreads();
+  }
+
+  // ---- phase 3: one thread per element: sums in the reference's order, SSP ----
+  if (tid < n)
+    element_sums<kNonlin, kSph, kTile>(A, tab, qs, qt, geo, res, tflag, wds, tbeg, info, slots, tid, tile0 + tid);
 }
 
 // slopelimiter.F:3300-3404: min/max of element means over each node's star,

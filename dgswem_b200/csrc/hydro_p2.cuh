@@ -577,10 +577,9 @@ __global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_consta
   const int ne = m.ne;
   const int tid = threadIdx.x;
   const int tile = blockIdx.x;
-  const int tile0 = m.tile_elem_ptr[tile];
-  const int n = m.tile_elem_ptr[tile + 1] - tile0;
-  const int hbeg = m.tile_halo_ptr[tile], nh = m.tile_halo_ptr[tile + 1] - hbeg;
-  const int tbeg = m.tile_task_ptr[tile], ntask = m.tile_task_ptr[tile + 1] - tbeg;
+  const int tile0 = tile * kP2Tile, n = min(kP2Tile, m.ne_tiled - tile0);
+  const int hbeg = tile * m.max_halo, nh = m.max_halo;
+  const int tbeg = tile * m.max_tasks, ntask = m.tile_count[tile].x;
   const P2Layout L = p2_layout(m.max_halo, m.max_tasks);
   P2EdgeBasis& B = *reinterpret_cast<P2EdgeBasis*>(smem_raw);
   real* qs = reinterpret_cast<real*>(smem_raw + L.qs);
@@ -623,6 +622,7 @@ __global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_consta
   for (int j = tid; j < kP2Tile + nh; j += kP2TileThreads) {
     if (j < kP2Tile && j >= n) continue;
     const int g = j < kP2Tile ? tile0 + j : (j == tid ? hg : m.tile_halo[hbeg + j - kP2Tile]);
+    if (g < 0) continue;
     real* sl = qs + j * kP2SlotStride;
 #ifdef DGSWEM_MIXED
     p2_slot_store(A, g, sl);  // FP32 values and the depth modes: through registers

@@ -9,8 +9,8 @@
 #define DGSWEM_VARIANT mixed
 #define DGSWEM_FAST_MATH 1
 #define DGSWEM_MIXED 1
-// FP32 terms need fewer registers and a smaller tile in shared memory:
-// 1152 resident stage threads per SM (three blocks of 384, 56 registers)
-#define DGSWEM_STAGE_RESIDENT_THREADS 1152
+// FP32 terms need fewer registers: 768 resident stage threads per SM (80
+// registers; 512 and 640 measure the same, shared memory holds five blocks)
+#define DGSWEM_STAGE_RESIDENT_THREADS 768
 #include "hydro_kernels.cuh"
 #include "kernel_launch.inc"

@@ -299,7 +299,7 @@ int dgswem_cuda_set_graph(dgswem_cuda* h, int steps);
 
 /* ---- tile and block shapes, autotuner ------------------------------------
  * The stage kernel is compiled for several tile shapes (elements per tile,
- * threads per block) and the limiter / WETDRY kernel for several block
+ * most edge tasks per tile) and the limiter / WETDRY kernel for several block
  * sizes; every shape gives bit-identical results.  dgswem_cuda_shapes lists
  * them (arrays of up to DGSWEM_CUDA_MAX_SHAPES entries, any may be NULL;
  * a limiter shape is its threads per block and the resident blocks per SM
