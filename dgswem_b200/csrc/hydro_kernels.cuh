@@ -73,6 +73,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 // all but the most recently committed group of this thread's copies complete
 __device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+// Programmatic dependent launch: the kernels of a stage are launched so that
+// each may start while the one before it ends.  Every thread passes chain_wait
+// before it reads or writes anything another kernel of the chain touches (what
+// comes before it reads only the mesh and the plan); chain_next lets the next
+// kernel's blocks in as this one's leave room.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async8_s(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
@@ -1098,9 +1105,11 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
         else
           cp_async4_s(gdst + rb * kStep * kTile * j, gsrc + j * step);
       }
-      if (r0 == 0) cp_async4(wds + w, A.wd + tile0 + w);
     }
   }
+  chain_wait();
+  chain_next();
+  if (tid < n) cp_async4(wds + tid, A.wd + tile0 + tid);
 #ifdef DGSWEM_MIXED
   // one thread per tile or halo element: its 12 FP64 values into registers,
   // then its FP32 slot (ZE, QX, QY modes and the depth modes ZE + HB, FP64
@@ -1204,10 +1213,13 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
 // sectors), and this pass writes three coalesced pair arrays.
 __global__ void node_minmax(const __grid_constant__ LimitArgs L) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p0 = n < L.m.np ? L.m.star_ptr[n] : 0, p1 = n < L.m.np ? L.m.star_ptr[n + 1] : 0;
+  chain_wait();
+  chain_next();
   if (n >= L.m.np) return;
   const int ne = L.m.ne;
   double zmin = 99999., zmax = -99999., xmin = 99999., xmax = -99999., ymin = 99999., ymax = -99999.;
-  for (int p = L.m.star_ptr[n]; p < L.m.star_ptr[n + 1]; ++p) {
+  for (int p = p0; p < p1; ++p) {
     const int e = L.m.star[p];
     const double zt = L.q[e], xt = L.q[(size_t)3 * ne + e], yt = L.q[(size_t)6 * ne + e];
     zmin = fmin(zmin, zt); xmin = fmin(xmin, xt); ymin = fmin(ymin, yt);
@@ -1251,11 +1263,15 @@ template <int kBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) limit_wetdry(const __grid_constant__ LimitArgs L) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = L.m.ne, np = L.m.np;
-  if (e >= L.ne_act) return;
   const BasisP1& B = cBasis;
-  int nd[3];
+  int nd[3] = {0, 0, 0};
+  if (e < L.ne_act) {
 #pragma unroll
-  for (int v = 0; v < 3; ++v) nd[v] = L.m.nm[(size_t)v * ne + e];
+    for (int v = 0; v < 3; ++v) nd[v] = L.m.nm[(size_t)v * ne + e];
+  }
+  chain_wait();
+  chain_next();
+  if (e >= L.ne_act) return;
   double q[9];
 #pragma unroll
   for (int c = 0; c < 9; ++c) q[c] = L.q[(size_t)c * ne + e];
