@@ -658,7 +658,7 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
   max_tasks = std::max(max_tasks, 1);
   if (max_halo + shape.tile > kMaxTileSlots || max_tasks >= (int)kNoTask)
     throw Failure(DGSWEM_ERR_ARG, "stage tile plan exceeds the task word's slot range");
-  const size_t stage_smem = stage_layout(shape.tile, max_halo, max_tasks, h->v->real_bytes).bytes;
+  const size_t stage_smem = stage_layout(shape.tile, max_halo, max_tasks, h->v->real_bytes, h->ph.nws != 0).bytes;
   int dev_smem = 0;
   DG_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
   if (stage_smem > (size_t)dev_smem)
@@ -1088,6 +1088,18 @@ void stage_forcing(const dgswem_cuda* h, double timedg, double rampdg, double* o
   }
 }
 
+// The form of a stage's SSP combination by its nonzero terms (SspKind)
+template <class Args>
+void ssp_kind(Args& A) {
+  const int irk = A.irk;
+  A.ca0 = A.a[0];
+  A.ca = A.a[irk - 1];
+  A.cb = A.b[irk - 1];
+  bool two = irk > 1 && A.a[0] != 0.0 && A.b[0] == 0.0;
+  for (int I = 1; I < irk - 1; ++I) two = two && A.a[I] == 0.0 && A.b[I] == 0.0;
+  A.ssp = A.ca == 0.0 || A.cb == 0.0 ? kSspAny : irk == 1 ? kSspOne : two ? kSspTwo : kSspAny;
+}
+
 // One RK stage: the stage kernel writes stage buffer irk for the owned
 // elements (launch_stage_rhs), then the limiter and WETDRY (launch_limit).
 // The p=2 stage: edge kernel, then element kernel (SSP combination included).
@@ -1111,6 +1123,7 @@ void launch_stage_p2(dgswem_cuda* h, int it, int irk, const double* forcing, con
     A.b[I - 1] = h->btvd[(size_t)(irk - 1) * nrk + (I - 1)] * h->dtdp;
   }
   A.rout = h->keep_rhs[irk - 1] ? h->rhs[irk - 1].p : nullptr;
+  ssp_kind(A);
   double timedg;
   stage_clock(h, it, irk, &timedg, &A.rampdg);
   A.ramp = ramp;
@@ -1160,14 +1173,7 @@ void launch_stage_rhs(dgswem_cuda* h, int it, int irk, const double* forcing, co
     A.b[I - 1] = h->btvd[(size_t)(irk - 1) * nrk + (I - 1)] * h->dtdp;
   }
   A.rout = h->keep_rhs[irk - 1] ? h->rhs[irk - 1].p : nullptr;
-  A.ca0 = A.a[0];
-  A.ca = A.a[irk - 1];
-  A.cb = A.b[irk - 1];
-  {
-    bool two = irk > 1 && A.a[0] != 0.0 && A.b[0] == 0.0;
-    for (int I = 1; I < irk - 1; ++I) two = two && A.a[I] == 0.0 && A.b[I] == 0.0;
-    A.ssp = A.ca == 0.0 || A.cb == 0.0 ? kSspAny : irk == 1 ? kSspOne : two ? kSspTwo : kSspAny;
-  }
+  ssp_kind(A);
   A.wd = h->wd.p;
   stage_clock(h, it, irk, &A.timedg, &A.rampdg);
   A.ramp = ramp;

@@ -183,13 +183,13 @@ constexpr unsigned kQStride = 14;
 constexpr unsigned kQfStride = 12;
 // Dynamic shared memory of the stage kernel (byte offsets)
 struct StageLayout {
-  unsigned qs, geo, qf, res, tab, wd, tflag, rare, bytes;
+  unsigned qs, geo, qf, met, res, tab, wd, tflag, rare, bytes;
 };
 __host__ __device__ inline unsigned align16(unsigned x) { return (x + 15u) & ~15u; }
 // tile: elements per tile of the shape; rb: bytes of the arithmetic type of
 // the edge and volume terms (8: FP64 kernels; 4: mixed precision, which adds
 // the FP32 slot copy qf)
-__host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int max_tasks, unsigned rb) {
+__host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int max_tasks, unsigned rb, bool nws) {
   StageLayout L;
   const unsigned nt = (unsigned)tile;
   const unsigned S = nt + (unsigned)max_halo;
@@ -201,7 +201,8 @@ __host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int 
   // the geometry rows kDrdx .. kSmemRows-1 of the tile, row r at geo + r * tile
   L.geo = rows - EGeo::kDrdx * nt * rb;
   L.qf = rows + (EGeo::kSmemRows - EGeo::kDrdx) * nt * rb;  // qf[S][kQfStride] (mixed only)
-  L.res = L.qf + (rb == 8u ? 0u : kQfStride * S * 4u);      // res[task][point][F, G, H], an odd stride
+  L.met = L.qf + (rb == 8u ? 0u : kQfStride * S * 4u);      // met[9][tile] (NWS only)
+  L.res = L.met + (nws ? 9u * nt * 8u : 0u);                // res[task][point][F, G, H], an odd stride
   L.tab = align16(L.res + 9u * T * rb);                     // BasisT::tr, sw
   L.wd = align16(L.tab + 54u * rb);                         // wd[S]
   L.tflag = align16(L.wd + S * 4u);                         // tflag[task]
@@ -329,6 +330,8 @@ struct P2Args {
   const double* rhist[kMaxStages];
   double* rout;
   double a[kMaxStages], b[kMaxStages];
+  int ssp;  // SspKind
+  double ca0, ca, cb;
   double rampdg;
   const double* __restrict__ ramp;  // RAMPDG in device memory (graph replays), or null: rampdg
   const double* __restrict__ ocean_zg;

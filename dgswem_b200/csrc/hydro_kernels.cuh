@@ -80,6 +80,22 @@ __device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.w
 // kernel's blocks in as this one's leave room.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launches a kernel of the chain: it may start before the one
+// ahead of it on the stream has ended.
+template <class Args>
+void launch_chained(void (*k)(Args), unsigned grid, unsigned block, size_t smem, cudaStream_t s, const Args& a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, a);
+}
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async8_s(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
@@ -630,7 +646,7 @@ __device__ __forceinline__ float manning_slow(float gn2, float depth) { return g
 // with one test that they are all in range at the end (ok).
 template <bool kNonlin, bool kSph, int kTile>
 __device__ __forceinline__ void volume_sums(const StageArgs& A, const BasisT<real>& C, const real q[12],
-                                            const real* geo, int el, int e, real rhs[3][3]) {
+                                            const real* geo, const double* met, int el, int e, real rhs[3][3]) {
   const MeshView& m = A.m;
   const Physics& P = A.ph;
   const PhysR R = phys_r(A);
@@ -743,10 +759,10 @@ __device__ __forceinline__ void volume_sums(const StageArgs& A, const BasisT<rea
         dpsidy[a] = drpsi[a] * drdy + dspsi[a] * dsdy;
       }
       const real fw = real(1) / f1, r = (real)stage_ramp(A);
-      const int n0 = m.nm[e], n1 = m.nm[(size_t)ne + e], n2 = m.nm[(size_t)2 * ne + e];
-      const real wx0 = r * (real)A.wsx[n0], wx1 = r * (real)A.wsx[n1], wx2 = r * (real)A.wsx[n2];
-      const real wy0 = r * (real)A.wsy[n0], wy1 = r * (real)A.wsy[n1], wy2 = r * (real)A.wsy[n2];
-      const real p0 = r * (real)A.pr[n0], p1 = r * (real)A.pr[n1], p2 = r * (real)A.pr[n2];
+      const double* w = met + el;  // rows wsx, wsy, pr of vertices 1, 2, 3
+      const real wx0 = r * (real)w[0], wx1 = r * (real)w[kTile], wx2 = r * (real)w[2 * kTile];
+      const real wy0 = r * (real)w[3 * kTile], wy1 = r * (real)w[4 * kTile], wy2 = r * (real)w[5 * kTile];
+      const real p0 = r * (real)w[6 * kTile], p1 = r * (real)w[7 * kTile], p2 = r * (real)w[8 * kTile];
       sx = sx + fw * (wx0 * C.psi[0][I] + wx1 * C.psi[1][I] + wx2 * C.psi[2][I]) -
            R.g * sfq * depth[I] * (p0 * dpsidx[0] + p1 * dpsidx[1] + p2 * dpsidx[2]);
       sy = sy + fw * (wy0 * C.psi[0][I] + wy1 * C.psi[1][I] + wy2 * C.psi[2][I]) -
@@ -870,7 +886,8 @@ __device__ __forceinline__ bool edge_task(const StageArgs& A, const real* tab, c
 // combination FP64).
 template <bool kNonlin, bool kSph, int kTile>
 __device__ __forceinline__ void element_sums(const StageArgs& A, const real* tab, const double* qs, const real* qt,
-                                             const real* geo, const real* res, const int* tflag, const int* wds,
+                                             const real* geo, const double* met, const real* res,
+                                             const int* tflag, const int* wds,
                                              int tbeg, unsigned info, unsigned slots, int el, int e) {
   const BasisT<real>& C = cBasisR;
   const MeshView& m = A.m;
@@ -994,7 +1011,7 @@ __device__ __forceinline__ void element_sums(const StageArgs& A, const real* tab
   if (wde != 0) {
     real q[12];
     slot_values(qt, el, q);
-    volume_sums<kNonlin, kSph, kTile>(A, C, q, geo, el, e, rhs);
+    volume_sums<kNonlin, kSph, kTile>(A, C, q, geo, met, el, e, rhs);
   }
   // SSP-RK combination (DG_hydro_timestep.F:238-290), zero coefficients
   // skipped: the stages whose nonzero terms are the current state and
@@ -1046,7 +1063,7 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
   const int tile0 = tile * kTile, n = min(kTile, m.ne_tiled - tile0);
   const int hbeg = tile * m.max_halo, tbeg = tile * m.max_tasks;
   const int2 count = m.tile_count[tile];  // tasks, those of them that read no halo element
-  const StageLayout L = stage_layout(kTile, m.max_halo, m.max_tasks, (unsigned)sizeof(real));
+  const StageLayout L = stage_layout(kTile, m.max_halo, m.max_tasks, (unsigned)sizeof(real), A.ph.nws != 0);
   double* qs = reinterpret_cast<double*>(smem_raw + L.qs);
   real* geo = reinterpret_cast<real*>(smem_raw + L.geo);
 #ifdef DGSWEM_MIXED
@@ -1058,6 +1075,7 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
   real* tab = reinterpret_cast<real*>(smem_raw + L.tab);  // BasisT::tr, then BasisT::sw
   int* wds = reinterpret_cast<int*>(smem_raw + L.wd);
   int* tflag = reinterpret_cast<int*>(smem_raw + L.tflag);
+  double* met = reinterpret_cast<double*>(smem_raw + L.met);  // nodal wind stress and pressure (NWS)
   int* rare = reinterpret_cast<int*>(smem_raw + L.rare);  // number, then ids, of the tasks left to edge_point_rare
 
   // ---- phase 1: tile and halo elements into shared memory ----
@@ -1106,6 +1124,11 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
           cp_async4_s(gdst + rb * kStep * kTile * j, gsrc + j * step);
       }
     }
+  }
+  int nd[3] = {0, 0, 0};
+  if (A.ph.nws != 0 && tid < n) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) nd[a] = m.nm[(size_t)a * ne + tile0 + tid];
   }
   chain_wait();
   chain_next();
@@ -1168,6 +1191,16 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
     }
   }
 
+  // the element's nodal wind stress and pressure, read in phase 3
+  if (A.ph.nws != 0 && tid < n) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      cp_async8(met + a * kTile + tid, A.wsx + nd[a]);
+      cp_async8(met + (3 + a) * kTile + tid, A.wsy + nd[a]);
+      cp_async8(met + (6 + a) * kTile + tid, A.pr + nd[a]);
+    }
+  }
+
   // ---- phase 2: one thread per edge task (the next round's task is fetched
   // while this one's is evaluated) ----
   for (int t0 = 0; t0 < count.x; t0 += kThreads) {
@@ -1187,6 +1220,7 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
         edge_task<kNonlin, kSph, kTile>(A, tab, qt, wds, tile0, hbeg, tk0, n0.x, n0.y, res + t * 9, tflag + t))
       rare[1 + atomicAdd(rare, 1)] = t;
   }
+  cp_async_wait_all();
   __syncthreads();
   // the tasks left out, a thread per (task, point): in any order, each writes
   // its own values
@@ -1203,7 +1237,7 @@ __global__ void __launch_bounds__(kThreads, stage_min_blocks(kThreads))
 
   // ---- phase 3: one thread per element: sums in the reference's order, SSP ----
   if (tid < n)
-    element_sums<kNonlin, kSph, kTile>(A, tab, qs, qt, geo, res, tflag, wds, tbeg, info, slots, tid, tile0 + tid);
+    element_sums<kNonlin, kSph, kTile>(A, tab, qs, qt, geo, met, res, tflag, wds, tbeg, info, slots, tid, tile0 + tid);
 }
 
 // slopelimiter.F:3300-3404: min/max of element means over each node's star,
@@ -1266,8 +1300,7 @@ __device__ __forceinline__ bool sweep_idle(const real vx[3], const real vmin[3],
 
 // slopelimiter.F:3555-3677: the three sweeps that restore the element mean z0
 __device__ __forceinline__ void sweeps(real vx[3], const real vmin[3], const real vmax[3], real z0) {
-  constexpr int kUnroll = sizeof(real) == 8 ? 1 : 3;
-#pragma unroll kUnroll
+#pragma unroll 1
   for (int sweep = 0; sweep < 3; ++sweep) {
     real sumdif;
     if (sweep_idle(vx, vmin, z0, sumdif)) break;

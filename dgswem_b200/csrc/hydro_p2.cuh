@@ -164,9 +164,12 @@ __device__ __forceinline__ P2Frc p2_force(const P2Args& A, int e) {
   return F;
 }
 
-template <bool kNonlin>
+// kTry: the reciprocal and roots without a branch, ok reset where an argument is
+// out of their range (see volume_sums); otherwise by the operators.
+template <bool kNonlin, bool kTry>
 __device__ __forceinline__ void p2_volume(const P2Args& A, const real* q, const real* w, real drdx, real dsdx,
-                                          real drdy, real dsdy, real hyb, const P2Frc& F, int i, real out[8]) {
+                                          real drdy, real dsdy, real hyb, const P2Frc& F, int i, real out[8],
+                                          bool& ok) {
   const Physics& P = A.ph;
   const PhysR R = phys_r(A);
   const BasisP2T<real>& C = cB2R;
@@ -209,7 +212,8 @@ __device__ __forceinline__ void p2_volume(const P2Args& A, const real* q, const 
   const real fx = uq * f1 * real(1), fy = vq * f1;
   const real fu = kNonlin ? uq : NLEQ * uq, fv = kNonlin ? vq : NLEQ * vq;
   const real fg = R.nleqg * zq * 1;
-  const real fh = real(1) / (kNonlin ? depth : NLEQ * depth + LEQ);
+  const real dq = kNonlin ? depth : NLEQ * depth + LEQ;
+  const real fh = kTry ? rcp_try(dq, ok) : rcp_slow(dq);
   const real u = uq * fh, v = vq * fh;
   const real huu = fu * u, hvv = fv * v, huv = fu * v;
   const real gh2 = kNonlin ? fg * (real(0.5) * zq + hq) : fg * (real(0.5) * zq + hq) + R.fg_l * zq;
@@ -217,15 +221,15 @@ __device__ __forceinline__ void p2_volume(const P2Args& A, const real* q, const 
   const real hx = huv * real(1), hy = hvv + gh2;
   if (A.m.manning) {
     const real nbar = F.nbar;
-    fric = R.g * (nbar * nbar) / cube_root(depth);
+    fric = kTry ? manning_try(R.g * (nbar * nbar), depth, ok) : manning_slow(R.g * (nbar * nbar), depth);
     if (fric < R.cf) fric = R.cf;
   }
   real tau = fric;
   if (P.iflinbf == 0) {
-    const real umag = sqrt(u * u + v * v);
+    const real umag = kTry ? sqrt_try(u * u + v * v, ok) : sqrt_slow(u * u + v * v);
     tau = tau * umag * fh;
     if (P.ifhybf == 1) tau = tau * hyb;
-    tau = fmin(tau, R.tau_cap);
+    tau = tau < R.tau_cap ? tau : R.tau_cap;
   }
   real sx = -(tau * uq) + fg * dhx * real(1) + cori * vq;
   real sy = -(tau * vq) + fg * dhy - cori * uq;
@@ -365,7 +369,8 @@ __global__ void __launch_bounds__(128, 4) p2_elements(const __grid_constant__ P2
   }
   for (int i = 0; i < kP2Agp; ++i) {
     real vol[8];
-    p2_volume<kNonlin>(A, q, wm, drdx, dsdx, drdy, dsdy, hyb, p2_force(A, e), i, vol);
+    bool ok;
+    p2_volume<kNonlin, false>(A, q, wm, drdx, dsdx, drdy, dsdy, hyb, p2_force(A, e), i, vol, ok);
     acc_t vw[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) vw[r] = vol[r];
@@ -422,25 +427,32 @@ __global__ void __launch_bounds__(128, 4) p2_elements(const __grid_constant__ P2
 // barriers:
 //   1. tile and halo elements' 24 slot values (18 modal values, six fourth-
 //      row modes: HB, or the depth modes in the mixed variant), the tile's
-//      geometry rows, edge info, task words and per-element forcing terms
-//      (P2Frc: Coriolis, friction, the vertices' wind and pressure) into
-//      shared memory, and the hybrid friction factor of each tile element;
-//   2. one work item per thread and round over the tile's edge points and
-//      then its area points: an edge point (edge task, Lobatto point) gives
-//      the LLF flux of the point in the reference's in/ex orientation, or the
-//      land / ocean ghost and its flux -> (F, G, H); an area point (element,
-//      point) gives its volume fluxes and sources;
-//   3. one thread per (element, mode): the mode's right-hand side of the
-//      three variables in the order of p2_elements (boundary edges, interior
-//      edges as the slot sum, rain, area points), then the SSP combination,
-//      its state operands loaded before the sums.
+//      geometry rows and per-element forcing terms (P2Frc: Coriolis, friction,
+//      the vertices' wind and pressure) into shared memory, and the hybrid
+//      friction factor of each tile element;
+//   2. one thread per edge task: the traces of both elements at the four
+//      Lobatto points, then the LLF flux of each in the reference's in/ex
+//      orientation -> (F, G, H); boundary tasks, and those with a value out of
+//      range of the straight-line reciprocals, after it, a thread per point;
+//      and one thread per (element, three area points): their volume fluxes
+//      and sources;
+//   3. one thread per (element, three modes): the modes' right-hand sides of
+//      the three variables in the order of p2_elements (boundary edges,
+//      interior edges as the slot sum, rain, area points), then the SSP
+//      combination.
+// Work is split so coarsely for the reasons given at stage_p1: 6,560 thread
+// instructions an element and stage (3,730 of them FP64) against 9,830 (3,840)
+// by point and mode, the area and sum loops rolled (unrolled they cost 5 % in
+// instruction fetches).  250k elements, strict: 147.8 -> 129.6 us a stage, two
+// blocks of 218 registers an SM 133.6, four of 128 149; mixed, 130k elements:
+// 64.8 -> 50.1 us.
 // Each interior edge point is evaluated once per tile (twice for an edge
 // between tiles) and its flux stays in shared memory: no flux slots in HBM.
 // Every sum has p2_elements' operands and order, so both give the same bits.
 // internal_edge_hydro.F, land_edge_hydro.F, ocean_edge_hydro.F,
 // rhs_dg_hydro.F, DG_hydro_timestep.F:238-290
 // ---------------------------------------------------------------------------
-constexpr int kP2Tile = 64, kP2TileThreads = 384;
+constexpr int kP2Tile = 64, kP2TileThreads = 128, kP2Blocks = 3;
 // slot stride in reals: 24 values and a pad keeping 16-byte loads by
 // consecutive slots off one bank group (13 or 7 16-byte units, odd)
 constexpr int kP2SlotStride = sizeof(real) == 8 ? 26 : 28;
@@ -449,30 +461,37 @@ constexpr int kP2Vol = 8;  // fx fy gx gy hx hy sx sy
 // stride spreads the tasks that a warp's elements read over the banks
 constexpr int kP2ResStride = 3 * kP2Egp + 1;
 
-// the edge traces' basis values, read with per-lane indices (local edge and
-// point vary across a warp) by the edge points, kept in shared memory with
-// rows of seven (the twelve (edge, point) rows a warp reads fall on
-// distinct banks); the sums read their edge weights from constant memory,
-// which takes that load off the shared-memory pipe
-constexpr int kP2EbRow = kP2Modes + 1;
-struct P2EdgeBasis {
-  real phi_edge[3][kP2Egp][kP2EbRow];
+// The tables read with per-lane indices (local edge and point vary across a
+// warp), kept in shared memory: the edge traces' basis values, modes 2..6 of a
+// point in a row of six (three 16-byte loads), and the sums' edge weights, in
+// the sums' type, in rows of seven (the twelve rows a warp reads fall on
+// distinct banks).
+#ifdef DGSWEM_MIXED
+using P2Acc = double;
+__device__ __forceinline__ const BasisP2& p2_acc_basis() { return cB2; }
+#else
+using P2Acc = real;
+__device__ __forceinline__ const BasisP2T<real>& p2_acc_basis() { return cB2R; }
+#endif
+struct P2Tables {
+  P2Acc edgeq[3][kP2Egp][kP2Modes + 1];
+  real phi[3][kP2Egp][kP2Modes];  // phi[..][k - 1]: mode k; one pad
 };
+__device__ P2Tables gP2Tab;
 
 struct P2Layout {
-  unsigned qs, geo, frc, vol, res, info, tasks, bytes;
+  unsigned qs, geo, frc, vol, res, rare, bytes;
 };
 __host__ __device__ inline P2Layout p2_layout(int max_halo, int max_tasks) {
   P2Layout L;
   const unsigned S = (unsigned)(kP2Tile + max_halo), T = (unsigned)max_tasks, rb = (unsigned)sizeof(real);
-  L.qs = align16((unsigned)sizeof(P2EdgeBasis));
+  L.qs = align16((unsigned)sizeof(P2Tables));
   L.geo = align16(L.qs + S * kP2SlotStride * rb);
   L.frc = align16(L.geo + kGeoRows * kP2Tile * rb);
   L.vol = align16(L.frc + P2Frc::kRows * kP2Tile * rb);
   L.res = align16(L.vol + kP2Vol * kP2Agp * kP2Tile * rb);
-  L.info = align16(L.res + T * kP2ResStride * rb);
-  L.tasks = align16(L.info + 2u * kP2Tile * 4u);
-  L.bytes = align16(L.tasks + T * 8u);
+  L.rare = align16(L.res + T * kP2ResStride * rb);
+  L.bytes = align16(L.rare + (T + 1u) * 4u);
   return L;
 }
 
@@ -487,12 +506,11 @@ __device__ __forceinline__ void p2_slot_store(const P2Args& A, int g, real* dst)
 
 // trace at point (led, gp) of the six modes at slot[off .. off+5], mode 1
 // first, as trace6 sums them
-template <class Basis>
-__device__ __forceinline__ real p2_slot_trace(const Basis& B, const real* slot, int off, int led, int gp) {
-  const real* phi = B.phi_edge[led][gp];
+__device__ __forceinline__ real p2_slot_trace(const P2Tables& B, const real* slot, int off, int led, int gp) {
+  const real* phi = B.phi[led][gp];
   real t = slot[off];
 #pragma unroll
-  for (int k = 1; k < kP2Modes; ++k) t = t + slot[off + k] * phi[k];
+  for (int k = 1; k < kP2Modes; ++k) t = t + slot[off + k] * phi[k - 1];
   return t;
 }
 
@@ -512,7 +530,7 @@ __device__ __forceinline__ real p2_hybrid(const Physics& P, const real* sl) {
 // flux in the in/ex orientation for an interior edge, else the land / ocean
 // ghost state and its flux
 template <bool kNonlin>
-__device__ __forceinline__ void p2_tile_edge_point(const P2Args& A, const P2EdgeBasis& B, const real* qs,
+__device__ __forceinline__ void p2_tile_edge_point(const P2Args& A, const P2Tables& B, const real* qs,
                                                    const real* geo, uint2 tk, int I, real* o) {
   const MeshView& m = A.m;
   const Physics& P = A.ph;
@@ -569,8 +587,41 @@ __device__ __forceinline__ void p2_tile_edge_point(const P2Args& A, const P2Edge
   o[0] = f.f; o[1] = f.g; o[2] = f.h;
 }
 
+// The traces of ZE, QX, QY and the fourth row of a slot at the four points of
+// local edge led (point p of `flip`ped sides is 3 - p), mode 1 first, as
+// trace6 sums them
+__device__ __forceinline__ void p2_traces(const P2Tables& B, const real* slot, int led, bool flip, real t[4][kP2Egp]) {
+  constexpr int kPer = 16 / (int)sizeof(real);
+  struct alignas(16) Vec {
+    real v[kPer];
+  };
+  const real* ph = B.phi[led][flip ? kP2Egp - 1 : 0];
+  const int step = flip ? -kP2Modes : kP2Modes;
+  real phi[kP2Egp][kP2Modes - 1];
+#pragma unroll
+  for (int p = 0; p < kP2Egp; ++p)
+#pragma unroll
+    for (int k = 0; k < kP2Modes - 1; ++k) phi[p][k] = ph[p * step + k];
+  real q[4 * kP2Modes];
+#pragma unroll
+  for (int i = 0; i < 4 * kP2Modes / kPer; ++i) {
+    const Vec x = reinterpret_cast<const Vec*>(slot)[i];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) q[i * kPer + j] = x.v[j];
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int p = 0; p < kP2Egp; ++p) {
+      real v = q[r * kP2Modes];
+#pragma unroll
+      for (int k = 1; k < kP2Modes; ++k) v = v + q[r * kP2Modes + k] * phi[p][k - 1];
+      t[r][p] = v;
+    }
+}
+
 template <bool kNonlin>
-__global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_constant__ P2Args A) {
+__global__ void __launch_bounds__(kP2TileThreads, kP2Blocks) p2_tile(const __grid_constant__ P2Args A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const MeshView& m = A.m;
   const Physics& P = A.ph;
@@ -581,26 +632,32 @@ __global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_consta
   const int hbeg = tile * m.max_halo, nh = m.max_halo;
   const int tbeg = tile * m.max_tasks, ntask = m.tile_count[tile].x;
   const P2Layout L = p2_layout(m.max_halo, m.max_tasks);
-  P2EdgeBasis& B = *reinterpret_cast<P2EdgeBasis*>(smem_raw);
+  P2Tables& B = *reinterpret_cast<P2Tables*>(smem_raw);
   real* qs = reinterpret_cast<real*>(smem_raw + L.qs);
   real* geo = reinterpret_cast<real*>(smem_raw + L.geo);
   real* frc = reinterpret_cast<real*>(smem_raw + L.frc);  // cori, fric, wx[3], wy[3], pr[3]: [kRows][kP2Tile]
   real* vol = reinterpret_cast<real*>(smem_raw + L.vol);
   real* res = reinterpret_cast<real*>(smem_raw + L.res);
-  unsigned* sinfo = reinterpret_cast<unsigned*>(smem_raw + L.info);  // [einfo | eslot][kP2Tile]
-  uint2* stasks = reinterpret_cast<uint2*>(smem_raw + L.tasks);
+  int* rare = reinterpret_cast<int*>(smem_raw + L.rare);  // number, then ids, of the tasks done point by point
   const real* G = egeo_r(m);
   const bool hybrid = P.iflinbf == 0 && P.ifhybf == 1;
-  for (int i = tid; i < 3 * kP2Egp * kP2Modes; i += kP2TileThreads) {
-    const int row = i / kP2Modes, k = i - row * kP2Modes;
-    (&B.phi_edge[0][0][0])[row * kP2EbRow + k] = (&cB2R.phi_edge[0][0][0])[i];
-  }
-  // ---- phase 1: slots, geometry rows, edge info, task words, forcing ----
-  // Exact copies go by cp.async (issued back to back, one wait); the halo
-  // ids are fetched first, the forcing gathers (node ids, then the nodal
-  // fields) last, so their round trips overlap the copies in flight.
+  const int half = tid / kP2Tile, el = tid - half * kP2Tile;  // of phases 2 and 3
+  // ---- phase 1: tables, geometry rows, slots, forcing ----
+  // Exact copies go by cp.async (issued back to back, one wait); what no kernel
+  // writes comes before the previous kernel's end.
+  static_assert(sizeof(P2Tables) % 4 == 0, "copied by words");
+  for (int i = tid; i < (int)sizeof(P2Tables) / 4; i += kP2TileThreads)
+    cp_async4(reinterpret_cast<int*>(smem_raw) + i, reinterpret_cast<const int*>(&gP2Tab) + i);
+  if (tid == 0) rare[0] = 0;
   const int hj = tid - kP2Tile;
   const int hg = (hj >= 0 && hj < nh) ? m.tile_halo[hbeg + hj] : -1;
+  uint2 tk = make_uint2(kIBarrier, 0u);
+  if (tid < m.max_tasks) tk = m.tile_tasks[tbeg + tid];
+  unsigned info = 0, slots = 0;
+  if (el < n) {
+    info = m.einfo[tile0 + el];
+    slots = m.eslot[tile0 + el];
+  }
   {
     constexpr unsigned rb = sizeof(real);
     const unsigned geo_s = smem_addr(geo);
@@ -614,11 +671,22 @@ __global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_consta
       }
     }
   }
-  if (tid < n) {
-    cp_async4(sinfo + tid, m.einfo + tile0 + tid);
-    cp_async4(sinfo + kP2Tile + tid, m.eslot + tile0 + tid);
+  // the forcing terms of the tile's elements, by the second half of the threads
+  // (written by no kernel: two round trips, node ids and nodal fields, that end
+  // before the state's copies do)
+  if (half == 1 && el < n) {
+    const P2Frc F = p2_force(A, tile0 + el);
+    frc[0 * kP2Tile + el] = F.cori;
+    frc[1 * kP2Tile + el] = F.fric;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      frc[(2 + a) * kP2Tile + el] = F.wx[a];
+      frc[(5 + a) * kP2Tile + el] = F.wy[a];
+      frc[(8 + a) * kP2Tile + el] = F.pr[a];
+    }
   }
-  for (int j = tid; j < ntask; j += kP2TileThreads) cp_async8(stasks + j, m.tile_tasks + tbeg + j);
+  chain_wait();
+  chain_next();
   for (int j = tid; j < kP2Tile + nh; j += kP2TileThreads) {
     if (j < kP2Tile && j >= n) continue;
     const int g = j < kP2Tile ? tile0 + j : (j == tid ? hg : m.tile_halo[hbeg + j - kP2Tile]);
@@ -634,39 +702,44 @@ __global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_consta
     for (int k = 0; k < kP2Modes; ++k) cp_async8_s(d + 8u * (3 * kP2Modes + k), m.hb + (size_t)k * ne + g);
 #endif
   }
-  {  // the last kP2Tile threads: the forcing terms of the tile's elements
-    const int j = tid - (kP2TileThreads - kP2Tile);
-    if (j >= 0 && j < n) {
-      const P2Frc F = p2_force(A, tile0 + j);
-      frc[0 * kP2Tile + j] = F.cori;
-      frc[1 * kP2Tile + j] = F.fric;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        frc[(2 + a) * kP2Tile + j] = F.wx[a];
-        frc[(5 + a) * kP2Tile + j] = F.wy[a];
-        frc[(8 + a) * kP2Tile + j] = F.pr[a];
-      }
-    }
-  }
   cp_async_wait_all();
   // hybrid friction factor of tile element tid from the slot it copied
   if (hybrid && tid < n) geo[SGeo::kHyb * kP2Tile + tid] = p2_hybrid<kNonlin>(P, qs + tid * kP2SlotStride);
   __syncthreads();
 
-  // ---- phase 2: edge points (edge task, Lobatto point), then area points ----
-  // (the edge items padded to whole warps: a warp's area points share the
-  // point i, so its basis values are uniform constant-memory loads)
-  const int nep = kP2Egp * ntask, nep_pad = (nep + 31) & ~31;
-  for (int w = tid; w < nep_pad + kP2Agp * kP2Tile; w += kP2TileThreads) {
-    if (w < nep_pad) {
-      if (w < nep) {
-        const int ti = w / kP2Egp, I = w - kP2Egp * ti;
-        p2_tile_edge_point<kNonlin>(A, B, qs, geo, stasks[ti], I, res + (size_t)ti * kP2ResStride + I * 3);
+  // ---- phase 2: edge tasks, then area points ----
+  for (int t = tid; t < ntask; t += kP2TileThreads) {
+    const uint2 tk0 = tk;
+    if (t + kP2TileThreads < ntask) tk = m.tile_tasks[tbeg + t + kP2TileThreads];
+    const unsigned fl = tk0.x;
+    bool ok = (fl & 7u) == kInterior;
+    if (ok) {
+      const int sin = (fl >> TaskBits::kInSlot) & 511, sex = (fl >> TaskBits::kExSlot) & 511;
+      const int led_in = (fl >> TaskBits::kLedIn) & 3, led_ex = (fl >> TaskBits::kLedEx) & 3;
+      const bool flip = (fl >> TaskBits::kFlip) & 1u;
+      const int owner = flip ? sex : sin, oled = flip ? led_ex : led_in;
+      real nx = geo[(EGeo::kNx + oled) * kP2Tile + owner], ny = geo[(EGeo::kNy + oled) * kP2Tile + owner];
+      if (flip) { nx = -nx; ny = -ny; }
+      real ti[4][kP2Egp], tx[4][kP2Egp];
+      p2_traces(B, qs + sin * kP2SlotStride, led_in, false, ti);
+      p2_traces(B, qs + sex * kP2SlotStride, led_ex, true, tx);
+      real* o = res + (size_t)t * kP2ResStride;
+#pragma unroll
+      for (int I = 0; I < kP2Egp; ++I) {
+        real hi, hti, hx, htx;
+        trace_depth<kNonlin>(P, ti[0][I], ti[3][I], hi, hti);
+        trace_depth<kNonlin>(P, tx[0][I], tx[3][I], hx, htx);
+        const Flux3T<real> f =
+            llf_ok<kNonlin, real, true>(P, ti[0][I], tx[0][I], ti[1][I], tx[1][I], ti[2][I], tx[2][I], hi, hx, hti,
+                                        htx, real(1), real(1), nx, ny, real(P.g), ok);
+        o[3 * I] = f.f;
+        o[3 * I + 1] = f.g;
+        o[3 * I + 2] = f.h;
       }
-      continue;
     }
-    const int wa = w - nep_pad, i = wa / kP2Tile, el = wa - i * kP2Tile;
-    if (el >= n) continue;
+    if (!ok) rare[1 + atomicAdd(rare, 1)] = t;
+  }
+  if (el < n) {
     const real* sl = qs + el * kP2SlotStride;
     real q[3 * kP2Modes], wm[kP2Modes];
 #pragma unroll
@@ -687,139 +760,180 @@ __global__ void __launch_bounds__(kP2TileThreads, 2) p2_tile(const __grid_consta
       F.wy[a] = met ? frc[(5 + a) * kP2Tile + el] : real(0);
       F.pr[a] = met ? frc[(8 + a) * kP2Tile + el] : real(0);
     }
-    real v[kP2Vol];
-    p2_volume<kNonlin>(A, q, wm, drdx, dsdx, drdy, dsdy, hyb, F, i, v);
+    bool ok = true;
+#pragma unroll 1
+    for (int j = 0; j < kP2Agp / 2; ++j) {
+      const int i = half * (kP2Agp / 2) + j;
+      real v[kP2Vol];
+      p2_volume<kNonlin, true>(A, q, wm, drdx, dsdx, drdy, dsdy, hyb, F, i, v, ok);
 #pragma unroll
-    for (int r = 0; r < kP2Vol; ++r) vol[(r * kP2Agp + i) * kP2Tile + el] = v[r];
+      for (int r = 0; r < kP2Vol; ++r) vol[(r * kP2Agp + i) * kP2Tile + el] = v[r];
+    }
+    if (__builtin_expect(!ok, 0)) {
+#pragma unroll 1
+      for (int j = 0; j < kP2Agp / 2; ++j) {
+        const int i = half * (kP2Agp / 2) + j;
+        real v[kP2Vol];
+        p2_volume<kNonlin, false>(A, q, wm, drdx, dsdx, drdy, dsdy, hyb, F, i, v, ok);
+#pragma unroll
+        for (int r = 0; r < kP2Vol; ++r) vol[(r * kP2Agp + i) * kP2Tile + el] = v[r];
+      }
+    }
   }
   __syncthreads();
-
-  // ---- phase 3: per (element, mode) sums in p2_elements' order, SSP ----
-  for (int w = tid; w < kP2Modes * kP2Tile; w += kP2TileThreads) {
-    const int K = w / kP2Tile, el = w - K * kP2Tile;
-    if (el >= n) continue;
-    const int e = tile0 + el;
-    // the SSP combination's state operands, loaded before the sums
-    const bool hist0 = A.irk > 1;
-    double qc[3], qh0[3], rh0[3];
-#pragma unroll
-    for (int V = 0; V < 3; ++V) {
-      const size_t c = (size_t)(kP2Modes * V + K) * ne + e;
-#ifdef DGSWEM_MIXED
-      qc[V] = A.qin[c];
-#else
-      qc[V] = qs[el * kP2SlotStride + kP2Modes * V + K];  // the slot holds qin exactly
-#endif
-      qh0[V] = (hist0 && A.a[0] != 0.0) ? A.qhist[0][c] : 0.0;
-      rh0[V] = (hist0 && A.b[0] != 0.0) ? A.rhist[0][c] : 0.0;
+  const int nrare = rare[0];
+  if (nrare > 0) {
+    for (int w = tid; w < kP2Egp * nrare; w += kP2TileThreads) {
+      const int t = rare[1 + w / kP2Egp], I = w % kP2Egp;
+      p2_tile_edge_point<kNonlin>(A, B, qs, geo, m.tile_tasks[tbeg + t], I, res + (size_t)t * kP2ResStride + I * 3);
     }
-    const unsigned info = sinfo[el], slots = sinfo[kP2Tile + el];
-    // The sums and their weights in FP64 in every variant: the mixed form
-    // rounds only the operands (fluxes, volume terms) to FP32.  With FP32
-    // weights the hydrostatic pressure's edge and volume integrals no longer
-    // cancel to FP32 precision, and on a fine mesh the residual drives a
-    // spurious flow (config 3 at 8M elements after 5000 steps: 1.5e-5 m,
-    // against 3.5e-6 m with FP64 weights and sums).
-#ifdef DGSWEM_MIXED
-    using acc_t = double;
-    const BasisP2& CW = cB2;
-#else
-    using acc_t = real;
-    const BasisP2T<real>& CW = cB2R;
-#endif
-    acc_t rhs[3] = {0, 0, 0}, isum[3] = {0, 0, 0};
+    __syncthreads();
+  }
+
+  // ---- phase 3: per (element, three modes) sums in p2_elements' order, SSP ----
+  if (el >= n) return;
+  const int e = tile0 + el, K0 = 3 * half;
+  // The sums and their weights in FP64 in every variant: the mixed form
+  // rounds only the operands (fluxes, volume terms) to FP32.  With FP32
+  // weights the hydrostatic pressure's edge and volume integrals no longer
+  // cancel to FP32 precision, and on a fine mesh the residual drives a
+  // spurious flow (config 3 at 8M elements after 5000 steps: 1.5e-5 m,
+  // against 3.5e-6 m with FP64 weights and sums).
+  using acc_t = P2Acc;
+  const auto& C = p2_acc_basis();
+  acc_t rhs[3][3], isum[3][3];  // [variable][mode - K0]
 #pragma unroll
+  for (int V = 0; V < 3; ++V)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { rhs[V][k] = 0; isum[V][k] = 0; }
+  const bool plain = (info & 0x1ffu) == 0u;  // three interior edges
+  auto add_edge = [&](int l) {
+    const bool is_in = ei_flag(info, l) != 0;
+    const real* r = res + (size_t)((slots >> (10 * l)) & kNoTask) * kP2ResStride;
+    const acc_t ed = geo[(EGeo::kEdfac + l) * kP2Tile + el];
+    const acc_t es = is_in ? -ed : ed;  // the in side subtracts: (-w) * v + acc equals acc - w * v exactly
+    acc_t acc[3][3];
+#pragma unroll
+    for (int I = 0; I < kP2Egp; ++I) {
+      const acc_t* w = &B.edgeq[l][is_in ? I : kP2Egp - 1 - I][K0];
+      const acc_t v[3] = {(acc_t)r[I * 3], (acc_t)r[I * 3 + 1], (acc_t)r[I * 3 + 2]};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const acc_t wk = es * w[k];
+#pragma unroll
+        for (int V = 0; V < 3; ++V) acc[V][k] = I == 0 ? mul_rn(wk, v[V]) : madd(wk, v[V], acc[V][k]);
+      }
+    }
+#pragma unroll
+    for (int V = 0; V < 3; ++V)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) isum[V][k] = isum[V][k] + acc[V][k];
+  };
+  if (__builtin_expect(plain, 1)) {
+#pragma unroll 1
+    for (int s = 0; s < 3; ++s) add_edge(ei_order(info, s));
+  } else {
+#pragma unroll 1
     for (int s = 0; s < 3; ++s) {
       const int l = ei_order(info, s);
       const unsigned kind = ei_kind(info, l);
       if (kind == kNone) continue;
-      const int ti = (slots >> (10 * l)) & kNoTask;
-      const real* r = res + (size_t)ti * kP2ResStride;
       if (kind == kInterior) {
-        const bool is_in = ei_flag(info, l) != 0;
-        const acc_t edfac = geo[(EGeo::kEdfac + l) * kP2Tile + el];
-        acc_t acc[3] = {0, 0, 0};
+        add_edge(l);
+        continue;
+      }
+      const real* r = res + (size_t)((slots >> (10 * l)) & kNoTask) * kP2ResStride;
+      const acc_t areas = G[(size_t)EGeo::kAreas * ne + e];
+      const acc_t xlen = G[(size_t)(EGeo::kXlen + l) * ne + e];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const acc_t wb = acc_t(2) * C.m_inv[K0 + k] / areas * xlen;
 #pragma unroll
         for (int I = 0; I < kP2Egp; ++I) {
-          const int j = is_in ? I : kP2Egp - 1 - I;
-          const acc_t wk = edfac * (acc_t)CW.edgeq[l][j][K];
-          // the in side subtracts: acc + (-wk) * v equals acc - wk * v exactly
-          const acc_t ws = is_in ? -wk : wk;
-          const acc_t v0 = r[I * 3], v1 = r[I * 3 + 1], v2 = r[I * 3 + 2];
-          acc[0] = acc[0] + ws * v0;
-          acc[1] = acc[1] + ws * v1;
-          acc[2] = acc[2] + ws * v2;
-        }
+          const acc_t wk = wb * C.phi_edge[l][I][K0 + k] * C.wegp[I];
 #pragma unroll
-        for (int V = 0; V < 3; ++V) isum[V] = isum[V] + acc[V];
-      } else {
-        const acc_t areas = G[(size_t)EGeo::kAreas * ne + e];
-        const acc_t xlen = G[(size_t)(EGeo::kXlen + l) * ne + e];
-#pragma unroll
-        for (int I = 0; I < kP2Egp; ++I) {
-          const acc_t wk = acc_t(2) * CW.m_inv[K] / areas * xlen * CW.phi_edge[l][I][K] * CW.wegp[I];
-          rhs[0] = rhs[0] - wk * (acc_t)r[I * 3];
-          rhs[1] = rhs[1] - wk * (acc_t)r[I * 3 + 1];
-          rhs[2] = rhs[2] - wk * (acc_t)r[I * 3 + 2];
+          for (int V = 0; V < 3; ++V) rhs[V][k] = madd(-wk, (acc_t)r[I * 3 + V], rhs[V][k]);
         }
       }
     }
+  }
 #pragma unroll
-    for (int V = 0; V < 3; ++V) rhs[V] = rhs[V] + isum[V];  // add_internal_flux
-    // the mode K and point i are the same across a warp: basis values from
-    // constant memory (uniform loads), the shared-memory pipe kept for the
-    // per-element operands
-    const auto& C = CW;
-    if (P.rainfall == 1) {
-      const acc_t src = acc_t(7.0556e-6);
-      for (int i = 0; i < kP2Agp; ++i) rhs[0] = rhs[0] + C.srfac[K][i] * src;
-    }
-    const acc_t drdx = geo[EGeo::kDrdx * kP2Tile + el], dsdx = geo[EGeo::kDsdx * kP2Tile + el];
-    const acc_t drdy = geo[EGeo::kDrdy * kP2Tile + el], dsdy = geo[EGeo::kDsdy * kP2Tile + el];
+  for (int V = 0; V < 3; ++V)
 #pragma unroll
-    for (int i = 0; i < kP2Agp; ++i) {
-      const real* vv = vol + i * kP2Tile + el;  // row r at vv[r * kP2Agp * kP2Tile]
-      const acc_t sx = vv[6 * kP2Agp * kP2Tile], sy = vv[7 * kP2Agp * kP2Tile];
-      if (K == 0) {
-        rhs[1] = rhs[1] + C.srfac[0][i] * sx;
-        rhs[2] = rhs[2] + C.srfac[0][i] * sy;
+    for (int k = 0; k < 3; ++k) rhs[V][k] = rhs[V][k] + isum[V][k];  // add_internal_flux
+  // the modes and points are the same across a warp: basis values from
+  // constant memory (uniform loads)
+  if (P.rainfall == 1) {
+    const acc_t src = acc_t(7.0556e-6);
+    for (int i = 0; i < kP2Agp; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) rhs[0][k] = rhs[0][k] + C.srfac[K0 + k][i] * src;
+  }
+  // the SSP combination's step-start state, in one batch, behind the area sums
+  double h0[9];
+  if (A.ssp == kSspTwo)
+#pragma unroll
+    for (int c = 0; c < 9; ++c) h0[c] = A.qhist[0][(size_t)(kP2Modes * (c / 3) + K0 + c % 3) * ne + e];
+  const acc_t drdx = geo[EGeo::kDrdx * kP2Tile + el], dsdx = geo[EGeo::kDsdx * kP2Tile + el];
+  const acc_t drdy = geo[EGeo::kDrdy * kP2Tile + el], dsdy = geo[EGeo::kDsdy * kP2Tile + el];
+#pragma unroll 1
+  for (int i = 0; i < kP2Agp; ++i) {
+    acc_t v[kP2Vol];
+#pragma unroll
+    for (int r = 0; r < kP2Vol; ++r) v[r] = vol[(r * kP2Agp + i) * kP2Tile + el];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int K = K0 + k;
+      const acc_t sr = C.srfac[K][i];
+      if (K == 0) {  // (warp-uniform: the first half of the threads)
+        rhs[1][k] = rhs[1][k] + sr * v[6];
+        rhs[2][k] = rhs[2][k] + sr * v[7];
       } else {
         const acc_t dpx = C.drphi[K][i] * drdx + C.dsphi[K][i] * dsdx;
         const acc_t dpy = C.drphi[K][i] * drdy + C.dsphi[K][i] * dsdy;
         const acc_t xf = C.mw[K][i] * dpx;
         const acc_t yf = C.mw[K][i] * dpy;
-        const acc_t sr = C.srfac[K][i];
-        rhs[0] = rhs[0] + xf * (acc_t)vv[0] + yf * (acc_t)vv[kP2Agp * kP2Tile];
-        rhs[1] = rhs[1] + xf * (acc_t)vv[2 * kP2Agp * kP2Tile] + yf * (acc_t)vv[3 * kP2Agp * kP2Tile] + sr * sx;
-        rhs[2] = rhs[2] + xf * (acc_t)vv[4 * kP2Agp * kP2Tile] + yf * (acc_t)vv[5 * kP2Agp * kP2Tile] + sr * sy;
+        rhs[0][k] = rhs[0][k] + xf * v[0] + yf * v[1];
+        rhs[1][k] = rhs[1][k] + xf * v[2] + yf * v[3] + sr * v[6];
+        rhs[2][k] = rhs[2][k] + xf * v[4] + yf * v[5] + sr * v[7];
       }
     }
-    // SSP-RK combination (DG_hydro_timestep.F:238-290) in FP64
-    bool bad = false;
-#pragma unroll
-    for (int V = 0; V < 3; ++V) {
-      const size_t c = (size_t)(kP2Modes * V + K) * ne + e;
-      const double rk = (double)rhs[V];
-      if (A.rout) A.rout[c] = rk;
-      double acc = 0.0;
-      if (hist0) {
-        if (A.a[0] != 0.0) acc = acc + A.a[0] * qh0[V];
-        if (A.b[0] != 0.0) acc = acc + A.b[0] * rh0[V];
-      }
-      for (int I = 1; I < A.irk; ++I) {
-        const bool cur = I == A.irk - 1;
-        if (A.a[I] != 0.0) acc = acc + A.a[I] * (cur ? qc[V] : A.qhist[I][c]);
-        if (A.b[I] != 0.0) acc = acc + A.b[I] * (cur ? rk : A.rhist[I][c]);
-      }
-      if (!hist0) {
-        if (A.a[0] != 0.0) acc = acc + A.a[0] * qc[V];
-        if (A.b[0] != 0.0) acc = acc + A.b[0] * rk;
-      }
-      bad = bad || isnan(acc);
-      A.qout[c] = acc;
-    }
-    if (bad) atomicOr(A.err, 1u);
   }
+  // SSP-RK combination (DG_hydro_timestep.F:238-290) in FP64
+  double out[9];
+  bool bad = false;
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    const int row = kP2Modes * (c / 3) + K0 + c % 3;
+    const size_t at = (size_t)row * ne + e;
+#ifdef DGSWEM_MIXED
+    const double qc = A.qin[at];
+#else
+    const double qc = qs[el * kP2SlotStride + row];  // the slot holds qin exactly
+#endif
+    const double rk = (double)rhs[c / 3][c % 3];
+    double acc = 0.0;
+    if (A.ssp != kSspAny) {
+      if (A.ssp == kSspTwo) acc = madd(A.ca0, h0[c], acc);
+      acc = madd(A.ca, qc, acc);
+      acc = madd(A.cb, rk, acc);
+    } else {
+      for (int I = 0; I < A.irk; ++I) {
+        const bool cur = I == A.irk - 1;
+        if (A.a[I] != 0.0) acc = acc + A.a[I] * (cur ? qc : A.qhist[I][at]);
+        if (A.b[I] != 0.0) acc = acc + A.b[I] * (cur ? rk : A.rhist[I][at]);
+      }
+    }
+    out[c] = acc;
+  }
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    const size_t at = (size_t)(kP2Modes * (c / 3) + K0 + c % 3) * ne + e;
+    bad = bad || isnan(out[c]);
+    A.qout[at] = out[c];
+    if (A.rout) A.rout[at] = (double)rhs[c / 3][c % 3];
+  }
+  if (bad) atomicOr(A.err, 1u);
 }
 
 // write_results.F:14-170 at p=2 (six modes at the element corners) + NODECODE
@@ -892,6 +1006,14 @@ void set_basis_p2(const BasisP2& b) {
   real* dst = reinterpret_cast<real*>(&r);
   for (size_t i = 0; i < sizeof(b) / sizeof(double); ++i) dst[i] = (real)src[i];
   cudaMemcpyToSymbol(cB2R, &r, sizeof(r));
+  P2Tables t{};
+  for (int l = 0; l < 3; ++l)
+    for (int j = 0; j < kP2Egp; ++j)
+      for (int k = 0; k < kP2Modes; ++k) {
+        t.edgeq[l][j][k] = (P2Acc)b.edgeq[l][j][k];
+        if (k > 0) t.phi[l][j][k - 1] = r.phi_edge[l][j][k];
+      }
+  cudaMemcpyToSymbol(gP2Tab, &t, sizeof(t));
 }
 
 void launch_p2_stage(const P2Args& a, bool nonlin, cudaStream_t s) {
@@ -899,7 +1021,7 @@ void launch_p2_stage(const P2Args& a, bool nonlin, cudaStream_t s) {
     const size_t smem = p2_layout(a.m.max_halo, a.m.max_tasks).bytes;
     auto* k = nonlin ? p2_tile<true> : p2_tile<false>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<(unsigned)a.ntile, kP2TileThreads, smem, s>>>(a);
+    launch_chained(k, (unsigned)a.ntile, kP2TileThreads, smem, s, a);
     return;
   }
   const unsigned ge = (unsigned)(((long long)kP2Egp * a.nedge + 127) / 128);
