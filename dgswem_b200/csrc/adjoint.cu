@@ -22,6 +22,7 @@
 // per-element buffer (one writer per slot); elem_vjp adds the volume terms
 // and gathers the buffer, so each element's outputs are written by its own
 // thread.
+#include "cr_math.cuh"
 #include "hydro_device.cuh"
 
 namespace dgswem {
@@ -29,11 +30,19 @@ namespace adj {
 
 __constant__ BasisP1 cB;
 
-void set_basis(const BasisP1& b) { cudaMemcpyToSymbol(cB, &b, sizeof(b)); }
+// the edge tables read with per-lane indices: PHI_EDGE, then EDGEQ; copied to
+// shared memory (constant loads by lane are replayed for each address)
+__device__ double gEdge[54];
+
+void set_basis(const BasisP1& b) {
+  cudaMemcpyToSymbol(cB, &b, sizeof(b));
+  static_assert(offsetof(BasisP1, phi_edge) == 0 && offsetof(BasisP1, edgeq) == sizeof(b.phi_edge), "gEdge");
+  cudaMemcpyToSymbol(gEdge, &b, sizeof(gEdge));
+}
 
 // Trace of ZE, QX, QY (q: 9 modal values) and HB (3) at edge point (led, j).
-__device__ __forceinline__ void trace(const double* q, const double* hb, int led, int j, double t[4]) {
-  const double p1 = cB.phi_edge[led][j][1], p2 = cB.phi_edge[led][j][2];
+__device__ __forceinline__ void trace(const double* q, const double* hb, const double* phi, double t[4]) {
+  const double p1 = phi[1], p2 = phi[2];
   t[0] = q[0] + q[1] * p1 + q[2] * p2;
   t[1] = q[3] + q[4] * p1 + q[5] * p2;
   t[2] = q[6] + q[7] * p1 + q[8] * p2;
@@ -43,11 +52,12 @@ __device__ __forceinline__ void trace(const double* q, const double* hb, int led
 // Reverse mode of the LLF flux (NLEQ=1, ICS=1) at in-side trace a and
 // ex-side trace b (ZE, QX, QY, HB each), normal (nx, ny), gravity G, given
 // the cotangent c of (F, G, H).  da, db receive the cotangents of the traces.
-__device__ void llf_vjp(const double a[4], const double b[4], double nx, double ny, double G, const double c[3],
+__device__ __forceinline__ void llf_vjp(const double a[4], const double b[4], double nx, double ny, double G, const double c[3],
                         double da[4], double db[4]) {
   const double* s[2] = {a, b};
   double* d[2] = {da, db};
   double H[2], iH[2], un[2], cc[2], aa[2];
+#pragma unroll
   for (int k = 0; k < 2; ++k) {
     H[k] = s[k][0] + s[k][3];
     iH[k] = 1.0 / H[k];
@@ -70,9 +80,12 @@ __device__ void llf_vjp(const double a[4], const double b[4], double nx, double 
   else if (eig == aa[0]) side = 0;
   else if (eig == aa[1] + cc[1]) { side = 1; with_c = true; }
   else side = 1;
-  double dun[2] = {0.0, 0.0}, dH[2] = {0.0, 0.0};
-  dun[side] += (un[side] >= 0.0 ? 1.0 : -1.0) * deig;
-  if (with_c && cc[side] > 0.0) dH[side] += G * (ny * ny + nx * nx) / (2.0 * cc[side]) * deig;
+  const double dus = ((side == 0 ? un[0] : un[1]) >= 0.0 ? 1.0 : -1.0) * deig, cs = side == 0 ? cc[0] : cc[1];
+  double dHs = 0.0;
+  if (with_c && cs > 0.0) dHs = G * (ny * ny + nx * nx) / (2.0 * cs) * deig;
+  const double dun[2] = {side == 0 ? dus : 0.0, side == 0 ? 0.0 : dus};
+  const double dH[2] = {side == 0 ? dHs : 0.0, side == 0 ? 0.0 : dHs};
+#pragma unroll
   for (int k = 0; k < 2; ++k) {
     const double z = s[k][0], qx = s[k][1], qy = s[k][2], h = s[k][3], r = iH[k];
     // F = 0.5 (qx nx + qy ny) summed over both sides
@@ -237,6 +250,52 @@ __device__ void volume_vjp(const AdjArgs& A, int e, int i, const double q[9], co
   }
 }
 
+// The reverse mode of an interior edge point with one dry side and a mass flux
+// F0 (internal_edge_hydro.F:212-302 with the forward's choice), out of line: its
+// arrays picked by side live in local memory.
+struct Trace4 {
+  double v[4];
+};
+struct Pair4 {
+  double a[4], b[4];
+};
+__device__ __noinline__ Pair4 front_vjp(Trace4 A4, Trace4 B4, double nx, double ny, double G, double F0, bool in_dry,
+                                        double cF, double cGi, double cHi, double cGx, double cHx) {
+  const double *ta = A4.v, *tb = B4.v;
+  double da[4] = {0, 0, 0, 0}, db[4] = {0, 0, 0, 0};
+  const bool refl = in_dry ? F0 > 0.0 : F0 < 0.0;
+  if (refl) {
+    // the wet side's state on both sides, its momentum reflected on the dry side
+    const double* w = in_dry ? tb : ta;
+    double rx, ry;
+    reflect(nx, ny, w[1], w[2], rx, ry);
+    const double wr[4] = {w[0], rx, ry, w[3]};
+    const double c[3] = {cF, in_dry ? cGx : cGi, in_dry ? cHx : cHi};
+    double dra[4], drb[4];
+    llf_vjp(in_dry ? wr : ta, in_dry ? tb : wr, nx, ny, G, c, dra, drb);
+    double* dw = in_dry ? db : da;
+    const double* dref = in_dry ? dra : drb;
+    const double* dself = in_dry ? drb : dra;
+    dw[0] += dself[0] + dref[0];
+    dw[3] += dself[3] + dref[3];
+    dw[1] += dself[1];
+    dw[2] += dself[2];
+    reflect_t(nx, ny, dref[1], dref[2], dw[1], dw[2]);
+  } else {
+    // F and the wet side's momentum flux from the flux at G; the dry
+    // side's momentum flux re-evaluated with G = 0
+    const double cf[3] = {cF, in_dry ? cGx : cGi, in_dry ? cHx : cHi};
+    const double cr[3] = {0.0, in_dry ? cGi : cGx, in_dry ? cHi : cHx};
+    double d1[4], d2[4], d3[4], d4[4];
+    llf_vjp(ta, tb, nx, ny, G, cf, d1, d2);
+    llf_vjp(ta, tb, nx, ny, 0.0, cr, d3, d4);
+    for (int k = 0; k < 4; ++k) { da[k] = d1[k] + d3[k]; db[k] = d2[k] + d4[k]; }
+  }
+  Pair4 r;
+  for (int k = 0; k < 4; ++k) { r.a[k] = da[k]; r.b[k] = db[k]; }
+  return r;
+}
+
 // Edge part: one thread per (edge, Lobatto point) of the edge list
 // A.edges (each interior edge once, from its in side, and each land / ocean
 // edge): the flux at that point is differentiated with respect to both
@@ -252,6 +311,11 @@ __device__ void volume_vjp(const AdjArgs& A, int e, int i, const double q[9], co
 __global__ void __launch_bounds__(256, 3) edge_vjp(const __grid_constant__ AdjArgs A) {
   const MeshView& m = A.m;
   const int ne = m.ne;
+  __shared__ double tab[54];
+  if (threadIdx.x < 54) tab[threadIdx.x] = gEdge[threadIdx.x];
+  chain_wait();
+  chain_next();
+  __syncthreads();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 3LL * A.nedge) return;
   const int ed = (int)(t / 3), I = (int)(t - 3LL * ed);
@@ -272,14 +336,14 @@ __global__ void __launch_bounds__(256, 3) edge_vjp(const __grid_constant__ AdjAr
       for (int c = 0; c < 9; ++c) { qi[c] = A.q[(size_t)c * ne + e]; qx[c] = A.q[(size_t)c * ne + ex]; }
       for (int k = 0; k < 3; ++k) { hi[k] = m.hb[(size_t)k * ne + e]; hx[k] = m.hb[(size_t)k * ne + ex]; }
       double ta[4], tb[4];
-      trace(qi, hi, l, I, ta);
-      trace(qx, hx, lx, 2 - I, tb);
+      trace(qi, hi, tab + (l * 3 + I) * 3, ta);
+      trace(qx, hx, tab + (lx * 3 + 2 - I) * 3, tb);
       const double efi = eg(EGeo::kEdfac + l, e), efx = eg(EGeo::kEdfac + lx, ex);
       // cotangents of F, G_in, H_in, G_ex, H_ex (the in side's sums subtract,
       // the ex side's add)
       double cF = 0, cGi = 0, cHi = 0, cGx = 0, cHx = 0;
       for (int k = 0; k < 3; ++k) {
-        const double wi_k = efi * cB.edgeq[l][I][k], wx_k = efx * cB.edgeq[lx][2 - I][k];
+        const double wi_k = efi * tab[27 + (l * 3 + I) * 3 + k], wx_k = efx * tab[27 + (lx * 3 + 2 - I) * 3 + k];
         cF += -wi_k * A.nu[(size_t)k * ne + e] + wx_k * A.nu[(size_t)k * ne + ex];
         cGi -= wi_k * A.nu[(size_t)(3 + k) * ne + e];
         cHi -= wi_k * A.nu[(size_t)(6 + k) * ne + e];
@@ -293,35 +357,10 @@ __global__ void __launch_bounds__(256, 3) edge_vjp(const __grid_constant__ AdjAr
         const double c[3] = {cF, cGi + cGx, cHi + cHx};
         llf_vjp(ta, tb, nx, ny, P.g, c, da, db);
       } else {  // internal_edge_hydro.F:212-302 with the forward's choice
-        const bool in_dry = wi == 0;
-        const bool refl = in_dry ? F0 > 0.0 : F0 < 0.0;
-        if (refl) {
-          // the wet side's state on both sides, its momentum reflected on the dry side
-          const double* w = in_dry ? tb : ta;
-          double rx, ry;
-          reflect(nx, ny, w[1], w[2], rx, ry);
-          const double wr[4] = {w[0], rx, ry, w[3]};
-          const double c[3] = {cF, in_dry ? cGx : cGi, in_dry ? cHx : cHi};
-          double dra[4], drb[4];
-          llf_vjp(in_dry ? wr : ta, in_dry ? tb : wr, nx, ny, P.g, c, dra, drb);
-          double* dw = in_dry ? db : da;
-          const double* dref = in_dry ? dra : drb;
-          const double* dself = in_dry ? drb : dra;
-          dw[0] += dself[0] + dref[0];
-          dw[3] += dself[3] + dref[3];
-          dw[1] += dself[1];
-          dw[2] += dself[2];
-          reflect_t(nx, ny, dref[1], dref[2], dw[1], dw[2]);
-        } else {
-          // F and the wet side's momentum flux from the flux at G; the dry
-          // side's momentum flux re-evaluated with G = 0
-          const double cf[3] = {cF, in_dry ? cGx : cGi, in_dry ? cHx : cHi};
-          const double cr[3] = {0.0, in_dry ? cGi : cGx, in_dry ? cHi : cHx};
-          double d1[4], d2[4], d3[4], d4[4];
-          llf_vjp(ta, tb, nx, ny, P.g, cf, d1, d2);
-          llf_vjp(ta, tb, nx, ny, 0.0, cr, d3, d4);
-          for (int k = 0; k < 4; ++k) { da[k] = d1[k] + d3[k]; db[k] = d2[k] + d4[k]; }
-        }
+        const Pair4 r = front_vjp(Trace4{ta[0], ta[1], ta[2], ta[3]}, Trace4{tb[0], tb[1], tb[2], tb[3]}, nx, ny, P.g,
+                                  F0, wi == 0, cF, cGi, cHi, cGx, cHx);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { da[k] = r.a[k]; db[k] = r.b[k]; }
       }
     }
     for (int k = 0; k < 4; ++k) { oi[k] = da[k]; ox[k] = db[k]; }
@@ -340,7 +379,7 @@ __global__ void __launch_bounds__(256, 3) edge_vjp(const __grid_constant__ AdjAr
   const int list = m.link[(size_t)l * ne + e];
   const double tx = -ny, ty = nx, den = 1.0 / (nx * ty - ny * tx);
   double ta[4], tb[4], c[3], da[4], db[4];
-  trace(q, hb, l, I, ta);
+  trace(q, hb, tab + (l * 3 + I) * 3, ta);
   tb[0] = ta[0]; tb[1] = ta[1]; tb[2] = ta[2]; tb[3] = ta[3];
   bool fixed = false;
   if (kind == kOcean) {
@@ -389,6 +428,8 @@ __global__ void __launch_bounds__(128, 5) elem_vjp(const __grid_constant__ AdjAr
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const MeshView& m = A.m;
   const int ne = m.ne;
+  chain_wait();
+  chain_next();
   if (e >= ne) return;
   double q[9], hb[3], nu[9], lam9[9], ghb[3] = {0, 0, 0}, gn = 0.0;
   for (int c = 0; c < 9; ++c) {
@@ -449,28 +490,35 @@ __global__ void __launch_bounds__(128, 5) elem_vjp(const __grid_constant__ AdjAr
 __global__ void node_arg(const MeshView m, const double* __restrict__ q, double* __restrict__ mm,
                          int* __restrict__ arg) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p0 = n < m.np ? m.star_ptr[n] : 0, p1 = n < m.np ? m.star_ptr[n + 1] : 0;
+  chain_wait();
+  chain_next();
   if (n >= m.np) return;
   const int ne = m.ne, np = m.np;
-  for (int var = 0; var < 3; ++var) {
-    double vmin = 99999., vmax = -99999.;
-    int amin = -1, amax = -1;
-    for (int p = m.star_ptr[n]; p < m.star_ptr[n + 1]; ++p) {
-      const int e = m.star[p];
+  double vmin[3] = {99999., 99999., 99999.}, vmax[3] = {-99999., -99999., -99999.};
+  int amin[3] = {-1, -1, -1}, amax[3] = {-1, -1, -1};
+  for (int p = p0; p < p1; ++p) {
+    const int e = m.star[p];
+#pragma unroll
+    for (int var = 0; var < 3; ++var) {
       const double t = q[(size_t)(3 * var) * ne + e];
-      if (t < vmin) { vmin = t; amin = e; }
-      if (t > vmax) { vmax = t; amax = e; }
+      if (t < vmin[var]) { vmin[var] = t; amin[var] = e; }
+      if (t > vmax[var]) { vmax[var] = t; amax[var] = e; }
     }
-    mm[(size_t)(2 * var) * np + n] = vmin;
-    mm[(size_t)(2 * var + 1) * np + n] = vmax;
-    arg[(size_t)(2 * var) * np + n] = amin;
-    arg[(size_t)(2 * var + 1) * np + n] = amax;
+  }
+#pragma unroll
+  for (int var = 0; var < 3; ++var) {
+    mm[(size_t)(2 * var) * np + n] = vmin[var];
+    mm[(size_t)(2 * var + 1) * np + n] = vmax[var];
+    arg[(size_t)(2 * var) * np + n] = amin[var];
+    arg[(size_t)(2 * var + 1) * np + n] = amax[var];
   }
 }
 
 __device__ __forceinline__ double div_count(double x, int kdp) {
   if (kdp <= 1) return x;
   if (kdp == 2) return x * 0.5;
-  return x / 3.0;
+  return div3(x);
 }
 
 // Reverse mode of WETDRY (wetdry.F:61-548) for element e with its branches
@@ -478,6 +526,25 @@ __device__ __forceinline__ double div_count(double x, int kdp) {
 // the cotangent of WETDRY's output to that of its input; ghb1 / ghb2 += the
 // terms of the flattening (ZE modes 2-3 set to -HB modes 2-3).  The nodal
 // depths DP are constants here.
+// Out of line: its arrays are indexed by the vertex order, in local memory.
+struct WetdryOut {
+  double lam[9], ghb1, ghb2;
+};
+struct Modes9 {
+  double v[9];
+};
+__device__ void wetdry_vjp(const MeshView& m, const Physics& ph, int e, int wd_in, const double q[9], double lam[9],
+                           double& ghb1, double& ghb2);
+__device__ __noinline__ WetdryOut wetdry_vjp_any(const MeshView& m, const Physics& ph, int e, int wd_in, Modes9 q,
+                                                 Modes9 lam) {
+  WetdryOut o;
+  double l[9];
+  for (int c = 0; c < 9; ++c) l[c] = lam.v[c];
+  o.ghb1 = o.ghb2 = 0.0;
+  wetdry_vjp(m, ph, e, wd_in, q.v, l, o.ghb1, o.ghb2);
+  for (int c = 0; c < 9; ++c) o.lam[c] = l[c];
+  return o;
+}
 __device__ void wetdry_vjp(const MeshView& m, const Physics& ph, int e, int wd_in, const double q[9], double lam[9],
                            double& ghb1, double& ghb2) {
   const int ne = m.ne;
@@ -578,9 +645,12 @@ __global__ void __launch_bounds__(128, 5) limit_vjp(const MeshView m, const Phys
                                                  double* __restrict__ lb, double* __restrict__ g_hb) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = m.ne, np = m.np;
+  int nd[3] = {0, 0, 0};
+  if (e < ne)
+    for (int v = 0; v < 3; ++v) nd[v] = m.nm[(size_t)v * ne + e];
+  chain_wait();
+  chain_next();
   if (e >= ne) return;
-  int nd[3];
-  for (int v = 0; v < 3; ++v) nd[v] = m.nm[(size_t)v * ne + e];
   double ql[9], l9[9];
   for (int c = 0; c < 9; ++c) {
     ql[c] = q[(size_t)c * ne + e];
@@ -604,7 +674,7 @@ __global__ void __launch_bounds__(128, 5) limit_vjp(const MeshView m, const Phys
         clamp[var][a] = vx[a] != c1 ? 2 : (c1 != v ? 1 : 0);
       }
       for (int w = 0; w < 3; ++w) {
-        const double sumloc = (vx[0] + vx[1] + vx[2]) / 3.0;
+        const double sumloc = div3(vx[0] + vx[1] + vx[2]);
         double sumdif = (sumloc - z[0]) * 3.0;
         const double s = copysign(1.0, sumdif);
         sgn[var][w] = s;
@@ -631,10 +701,24 @@ __global__ void __launch_bounds__(128, 5) limit_vjp(const MeshView m, const Phys
     }
   }
   if (wetdry != 0) {
-    double g1 = 0.0, g2 = 0.0;
-    wetdry_vjp(m, ph, e, wd[e], ql, l9, g1, g2);
-    g_hb[(size_t)ne + e] += g1;
-    g_hb[(size_t)2 * ne + e] += g2;
+    // a wet element with three wet vertices is left as it is
+    const int wd_in = wd[e];
+    bool plain = wd_in == 1;
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+      const double zn = ql[0] + cB.phi_corner[v][1] * ql[1] + cB.phi_corner[v][2] * ql[2];
+      plain = plain && !(m.dp[nd[v]] + zn <= ph.h0 + 1.0e-6);
+    }
+    if (!plain) {
+      Modes9 a, b;
+#pragma unroll
+      for (int c = 0; c < 9; ++c) { a.v[c] = ql[c]; b.v[c] = l9[c]; }
+      const WetdryOut o = wetdry_vjp_any(m, ph, e, wd_in, a, b);
+#pragma unroll
+      for (int c = 0; c < 9; ++c) l9[c] = o.lam[c];
+      g_hb[(size_t)ne + e] += o.ghb1;
+      g_hb[(size_t)2 * ne + e] += o.ghb2;
+    }
   }
   if (slopeflag != 0) {
     for (int var = 0; var < 3; ++var) {
@@ -681,10 +765,13 @@ __global__ void __launch_bounds__(128, 5) limit_vjp(const MeshView m, const Phys
 // Per node: the cotangents of its bounds, summed over its star in star order.
 __global__ void node_bound_gather(const MeshView m, const double* __restrict__ lb, double* __restrict__ nb) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p0 = n < m.np ? m.star_ptr[n] : 0, p1 = n < m.np ? m.star_ptr[n + 1] : 0;
+  chain_wait();
+  chain_next();
   if (n >= m.np) return;
   const int ne = m.ne, np = m.np;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int p = m.star_ptr[n]; p < m.star_ptr[n + 1]; ++p) {
+  for (int p = p0; p < p1; ++p) {
     const int e = m.star[p];
     const int a = m.nm[e] == n ? 0 : (m.nm[(size_t)ne + e] == n ? 1 : 2);
     for (int var = 0; var < 3; ++var) {
@@ -701,12 +788,18 @@ __global__ void elem_bound_scatter(const MeshView m, const int* __restrict__ arg
                                    double* __restrict__ lam) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = m.ne, np = m.np;
+  int nd[3] = {0, 0, 0};
+  if (e < ne)
+    for (int v = 0; v < 3; ++v) nd[v] = m.nm[(size_t)v * ne + e];
+  chain_wait();
+  chain_next();
   if (e >= ne) return;
   double add[3] = {0, 0, 0};
+#pragma unroll
   for (int v = 0; v < 3; ++v) {
-    const int n = m.nm[(size_t)v * ne + e];
-    if (v == 1 && n == m.nm[e]) continue;  // a node listed twice counts once
-    if (v == 2 && (n == m.nm[e] || n == m.nm[(size_t)ne + e])) continue;
+    const int n = nd[v];
+    if (v == 1 && n == nd[0]) continue;  // a node listed twice counts once
+    if (v == 2 && (n == nd[0] || n == nd[1])) continue;
     for (int r = 0; r < 6; ++r)
       if (arg[(size_t)r * np + n] == e) add[r / 2] += nb[(size_t)r * np + n];
   }
@@ -717,11 +810,11 @@ void launch_limit_vjp(const MeshView& m, const Physics& ph, int slopeflag, int w
                       const double* qpre, double* mm, int* arg, double* lam, double* lb, double* nb, double* g_hb,
                       cudaStream_t s) {
   const unsigned gn = (unsigned)((m.np + 127) / 128), ge = (unsigned)((m.ne + 127) / 128);
-  if (slopeflag != 0) node_arg<<<gn, 128, 0, s>>>(m, qpre, mm, arg);
-  limit_vjp<<<ge, 128, 0, s>>>(m, ph, slopeflag, wetdry, wd, qpre, mm, lam, lb, g_hb);
+  if (slopeflag != 0) launch_chained(node_arg, gn, 128, 0, s, m, qpre, mm, arg);
+  launch_chained(limit_vjp, ge, 128, 0, s, m, ph, slopeflag, wetdry, wd, qpre, mm, lam, lb, g_hb);
   if (slopeflag != 0) {
-    node_bound_gather<<<gn, 128, 0, s>>>(m, lb, nb);
-    elem_bound_scatter<<<ge, 128, 0, s>>>(m, arg, nb, lam);
+    launch_chained(node_bound_gather, gn, 128, 0, s, m, lb, nb);
+    launch_chained(elem_bound_scatter, ge, 128, 0, s, m, arg, nb, lam);
   }
 }
 
@@ -729,6 +822,8 @@ void launch_limit_vjp(const MeshView& m, const Physics& ph, int slopeflag, int w
 // (first: lam_I = a_I lam_j, nu_I = b_I lam_j)
 __global__ void ssp_adj(const __grid_constant__ SspAdjArgs A) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
+  chain_next();
   if (i >= A.len) return;
   const double l = A.lam_j[i];
   if (A.first) {
@@ -747,6 +842,8 @@ __global__ void ssp_adj(const __grid_constant__ SspAdjArgs A) {
 __global__ void gauge_eval(const double* __restrict__ q, int ne, const int* __restrict__ elem,
                            const double* __restrict__ phi, int ng, double* __restrict__ eta) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
+  chain_next();
   if (g >= ng) return;
   const int e = elem[g];
   eta[g] = phi[3 * g] * q[e] + phi[3 * g + 1] * q[(size_t)ne + e] + phi[3 * g + 2] * q[(size_t)2 * ne + e];
@@ -758,6 +855,8 @@ __global__ void gauge_seed(double* lam, int ne, const int* __restrict__ gel, con
                            const int* __restrict__ ggauge, const double* __restrict__ phi,
                            const double* __restrict__ w, int ngroup) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
+  chain_next();
   if (t >= ngroup) return;
   double a0 = 0.0, a1 = 0.0, a2 = 0.0;
   for (int i = gptr[t]; i < gptr[t + 1]; ++i) {
@@ -774,25 +873,25 @@ __global__ void gauge_seed(double* lam, int ne, const int* __restrict__ gel, con
 
 void launch_rhs_vjp(const AdjArgs& a, cudaStream_t s) {
   if (a.m.ne <= 0) return;
-  if (a.nedge > 0) edge_vjp<<<(unsigned)((3LL * a.nedge + 255) / 256), 256, 0, s>>>(a);
-  elem_vjp<<<(unsigned)((a.m.ne + 127) / 128), 128, 0, s>>>(a);
+  if (a.nedge > 0) launch_chained(edge_vjp, (unsigned)((3LL * a.nedge + 255) / 256), 256, 0, s, a);
+  launch_chained(elem_vjp, (unsigned)((a.m.ne + 127) / 128), 128, 0, s, a);
 }
 
 void launch_ssp_adj(const SspAdjArgs& a, cudaStream_t s) {
   if (a.len <= 0 || a.n <= 0) return;
-  ssp_adj<<<(unsigned)((a.len + 255) / 256), 256, 0, s>>>(a);
+  launch_chained(ssp_adj, (unsigned)((a.len + 255) / 256), 256, 0, s, a);
 }
 
 void launch_gauge_eval(const double* q, int ne, const int* elem, const double* phi, int ng, double* eta,
                        cudaStream_t s) {
   if (ng <= 0) return;
-  gauge_eval<<<(unsigned)((ng + 127) / 128), 128, 0, s>>>(q, ne, elem, phi, ng, eta);
+  launch_chained(gauge_eval, (unsigned)((ng + 127) / 128), 128, 0, s, q, ne, elem, phi, ng, eta);
 }
 
 void launch_gauge_seed(double* lam, int ne, const int* gel, const int* gptr, const int* ggauge, const double* phi,
                        const double* w, int ngroup, cudaStream_t s) {
   if (ngroup <= 0) return;
-  gauge_seed<<<(unsigned)((ngroup + 127) / 128), 128, 0, s>>>(lam, ne, gel, gptr, ggauge, phi, w, ngroup);
+  launch_chained(gauge_seed, (unsigned)((ngroup + 127) / 128), 128, 0, s, lam, ne, gel, gptr, ggauge, phi, w, ngroup);
 }
 
 }  // namespace adj

@@ -211,6 +211,32 @@ __host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int 
   return L;
 }
 
+#if defined(__CUDACC__)
+// Programmatic dependent launch: the kernels of a stage are launched so that
+// each may start while the one before it ends.  Every thread passes chain_wait
+// before it reads or writes anything another kernel of the chain touches (what
+// comes before it reads only the mesh and the plan); chain_next lets the next
+// kernel's blocks in as this one's leave room.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launches a kernel of the chain: it may start before the one
+// ahead of it on the stream has ended.
+template <class... P, class... Args>
+void launch_chained(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, Args&&... a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+}
+#endif
+
 struct Physics {
   double g, h0, dtdp, nleq, leq, nleqg, fg_l;
   double tau_cap;  // .9 * (1 / DTDP), the friction cap of rhs_dg_hydro.F

@@ -73,29 +73,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 // all but the most recently committed group of this thread's copies complete
 __device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-// Programmatic dependent launch: the kernels of a stage are launched so that
-// each may start while the one before it ends.  Every thread passes chain_wait
-// before it reads or writes anything another kernel of the chain touches (what
-// comes before it reads only the mesh and the plan); chain_next lets the next
-// kernel's blocks in as this one's leave room.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Launches a kernel of the chain: it may start before the one
-// ahead of it on the stream has ended.
-template <class Args>
-void launch_chained(void (*k)(Args), unsigned grid, unsigned block, size_t smem, cudaStream_t s, const Args& a) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, a);
-}
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async8_s(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
