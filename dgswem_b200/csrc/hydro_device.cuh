@@ -134,10 +134,13 @@ constexpr TileShape kTileShapes[kNumTileShapes] = {{128, 384, 128}, {64, 192, 64
 constexpr int kDefaultTileShape = 0;
 // Block sizes of the limiter / WETDRY element kernel (limit_wetdry), each
 // compiled for 1024 resident threads per SM except the last (768: more
-// registers per thread)
+// registers per thread).  The default is the smallest block: each warp works by
+// itself, and a block's registers are held until its slowest warp has swept
+// (1M elements under waves, blocks of 256 / 128 / 64: 61.4 / 59.0 / 58.4 us;
+// ensemble of 760k elements, mixed build: 36.3 us in blocks of 256, 35.0 of 64).
 constexpr int kNumLimitShapes = 3;
-constexpr int kLimitBlocks[kNumLimitShapes] = {256, 128, 256};
-constexpr int kLimitMinBlocks[kNumLimitShapes] = {4, 8, 3};
+constexpr int kLimitBlocks[kNumLimitShapes] = {64, 128, 256};
+constexpr int kLimitMinBlocks[kNumLimitShapes] = {16, 8, 3};
 constexpr int kDefaultLimitShape = 0;
 constexpr unsigned kNoTask = 1023u;
 constexpr int kMaxTileSlots = 512;  // tile + halo rows addressable by a task word's 9-bit slots

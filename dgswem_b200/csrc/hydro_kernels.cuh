@@ -1253,15 +1253,6 @@ __device__ __forceinline__ double2 node_bounds(const double* minmax, int np, int
 __device__ __forceinline__ double third_of(double x) { return div3(x); }
 __device__ __forceinline__ float third_of(float x) { return x / 3.0f; }
 
-// x / d for the redistribution divisor d = max(1, kdp) in {1, 2, 3}: x / 1
-// and x / 2 are exact scalings (x * 0.5 is the same correctly rounded value
-// as x / 2), x / 3 the correctly rounded quotient.
-__device__ __forceinline__ real div_count(real x, int kdp) {
-  if (kdp <= 1) return x;
-  if (kdp == 2) return x * real(0.5);
-  return third_of(x);
-}
-
 // Whether a redistribution sweep of vertex values vx about the mean z0 would
 // start from sumdif == +0 with every vx - vmin free of a sign bit: such a sweep
 // changes no bit, as each redfac is +0 (the quotient of +0, or 0, capped by a
@@ -1285,18 +1276,26 @@ __device__ __forceinline__ void sweeps(real vx[3], const real vmin[3], const rea
     real dif[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) dif[a] = (vx[a] - z0) * signdif;
-    int kdp = (dif[0] > 0) + (dif[1] > 0) + (dif[2] > 0);
+    // sumdif is shared out over the vertices left with dif > 0, the next vertex
+    // included: a third if all three have it, else a half or all of it (exact
+    // scalings).  As selects: the branches on that count left a warp's 32 pairs
+    // a few lanes at a time.  Only the third, a division, stays a branch.
+    const bool up0 = dif[0] > 0, up1 = dif[1] > 0, up2 = dif[2] > 0, pos = signdif > 0;
+    real first = sumdif * signdif;
+    if (up0 && up1 && up2)
+      first = third_of(first);
+    else
+      first = first * (up1 || up2 ? real(0.5) : real(1));
+    const real half = up2 ? real(0.5) : real(1);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      real redfac = 0;
-      if (dif[k] > 0) {  // sumdif * signdif / max(1, kdp)
-        redfac = div_count(sumdif * signdif, kdp);
-        kdp = kdp - 1;
-      }
-      const real redmax = signdif > 0 ? vx[k] - vmin[k] : vmax[k] - vx[k];
+      real redfac = k == 0 ? first : k == 1 ? sumdif * signdif * half : sumdif * signdif;
+      if (!(k == 0 ? up0 : k == 1 ? up1 : up2)) redfac = 0;
+      const real redmax = pos ? vx[k] - vmin[k] : vmax[k] - vx[k];
       redfac = fmin(redfac, redmax);
-      sumdif = sumdif - redfac * signdif;
-      vx[k] = vx[k] - redfac * signdif;
+      const real red = redfac * signdif;
+      sumdif = sumdif - red;
+      vx[k] = vx[k] - red;
     }
   }
 }
@@ -1311,9 +1310,10 @@ __device__ __forceinline__ void sweeps(real vx[3], const real vmin[3], const rea
 // to nine sweeps (1,480 warp against 720 thread instructions an element).  So a
 // warp of the FP64 builds first clamps all three variables, collects the pairs
 // that need sweeps in shared memory, and then sweeps them 32 at a time: 68.0 ->
-// 61.4 us on 1M elements, 1,260 warp instructions.  The mixed variant, which
-// sweeps only clamped variables, keeps them in place (34.9 us against 36.1 on
-// 760k elements).
+// 61.4 us on 1M elements, 1,260 warp instructions; 56.2 us with the sweep's
+// shares as selects and blocks of 64.  The mixed variant, which sweeps only
+// clamped variables, keeps them in place (34.9 us against 36.1 on 760k
+// elements; 32.3 with the selects).
 // Compiled per limiter shape (kLimitBlocks / kLimitMinBlocks).
 constexpr int kLimitPairs = 96;  // (element, variable) pairs of a warp
 template <int kBlock, int kMinBlocks>
