@@ -78,9 +78,9 @@ STEP_BYTES_PER_ELEMENT_STAGE = STAGE_KERNEL_BYTES + 12 + 24
 STAGE_OVERHEAD_BYTES = {"geometry_rows_beyond_model": 112 - 48, "tile_plan": 14, "edge_info": 8}
 # DRAM bytes per element of one stage_p1 launch (strict build),
 # dram__bytes_read.sum + dram__bytes_write.sum from ncu on the same deck at
-# 999,492 elements: the mean of a stage-1 (292.2) and a stage-2 (368.6)
+# 999,192 elements: the mean of a stage-1 (270.9) and a stage-2 (346.5)
 # launch; traffic grows with the element count.
-STAGE_TRAFFIC_BYTES = 0.5 * (292.2 + 368.6)
+STAGE_TRAFFIC_BYTES = 0.5 * (270.9 + 346.5)
 
 
 def rank_env():
@@ -983,7 +983,7 @@ def main(argv=None):
         "roofline": {"bound": "hbm", "kernel": "stage_p1", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": STAGE_TRAFFIC_BYTES * ne,
-                     "traffic_source": "ncu dram bytes per element of a stage-1 and a stage-2 launch (999,492 elements), "
+                     "traffic_source": "ncu dram bytes per element of a stage-1 and a stage-2 launch (999,192 elements), "
                                        "scaled by the element count",
                      "algorithmic_bytes_per_element_stage": STAGE_KERNEL_BYTES,
                      "overhead_bytes_per_element_stage": STAGE_OVERHEAD_BYTES,
