@@ -167,8 +167,14 @@ __device__ __forceinline__ void side_terms(float di, float de, float si, float s
   ci = sqrtf(si);
   ce = sqrtf(se);
 }
-// fmax without the NaN handling of FP64's (no maximum instruction)
-__device__ __forceinline__ double larger(double a, double b) { return a > b ? a : b; }
+// The larger speed of an edge point's two sides, skipping a NaN one (a side of
+// depth zero without flow: its mass flux still takes the other side's speed).
+// kTry: by one comparison, without FP64 fmax's NaN handling: a NaN speed needs a
+// depth or a discharge for which side_terms resets ok, or that leaves no flux
+// finite.
+template <bool kTry>
+__device__ __forceinline__ double larger(double a, double b) { return kTry ? (a > b ? a : b) : fmax(a, b); }
+template <bool kTry>
 __device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
 
 // numerical_flux.F:750-914, Local Lax-Friedrichs, in arithmetic type T.
@@ -231,7 +237,7 @@ __device__ __forceinline__ Flux3T<T> llf_ok(const Physics& P, T ze_in, T ze_ex, 
   // |un| + c equals the rounded larger of |un + c| and |un - c| exactly, so
   // fmax(|un| + c, |un|) is the same value; with c = NaN (negative depth) both
   // forms reduce to |un|, as fmax skips NaN operands.
-  const T eig = larger(side_speed(fabs(uni), ci), side_speed(fabs(une), ce));
+  const T eig = larger<kTry>(side_speed(fabs(uni), ci), side_speed(fabs(une), ce));
   Flux3T<T> r;
   r.f = f1a - T(0.5) * eig * j1;
   if (kNonlin) {
