@@ -254,7 +254,7 @@ __device__ __forceinline__ Flux3T<T> llf_ok(const Physics& P, T ze_in, T ze_ex, 
 template <bool kNonlin, class T>
 __device__ __forceinline__ Flux3T<T> llf(const Physics& P, T ze_in, T ze_ex, T qx_in, T qx_ex, T qy_in, T qy_ex,
                                          T hb_in, T hb_ex, T ht_in, T ht_ex, T sf_in, T sf_ex, T nx, T ny, T G) {
-  bool ok;
+  bool ok = true;
   return llf_ok<kNonlin, T>(P, ze_in, ze_ex, qx_in, qx_ex, qy_in, qy_ex, hb_in, hb_ex, ht_in, ht_ex, sf_in, sf_ex,
                             nx, ny, G, ok);
 }

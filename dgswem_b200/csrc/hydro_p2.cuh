@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(128, 4) p2_elements(const __grid_constant__ P2
   }
   for (int i = 0; i < kP2Agp; ++i) {
     real vol[8];
-    bool ok;
+    bool ok = true;
     p2_volume<kNonlin, false>(A, q, wm, drdx, dsdx, drdy, dsdy, hyb, p2_force(A, e), i, vol, ok);
     acc_t vw[8];
 #pragma unroll
