@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(128, 5) elem_vjp(const __grid_constant__ AdjAr
 
 // Node min / max of the element means (as node_minmax) and the first star
 // element attaining each: arg[(2 var + {0 min, 1 max}) * NP + n].
-__global__ void node_arg(const MeshView m, const double* __restrict__ q, double* __restrict__ mm,
+__global__ void node_arg(const MeshView m, const double* q, double* __restrict__ mm,
                          int* __restrict__ arg) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const int p0 = n < m.np ? m.star_ptr[n] : 0, p1 = n < m.np ? m.star_ptr[n + 1] : 0;
@@ -640,8 +640,8 @@ __device__ void wetdry_vjp(const MeshView& m, const Physics& ph, int e, int wd_i
 // (without the bound terms); lb[e*18 + (var*3 + a)*2 + {0 min, 1 max}]: the
 // cotangent of vertex a's bounds; g_hb += WETDRY's HB terms.
 __global__ void __launch_bounds__(128, 5) limit_vjp(const MeshView m, const Physics ph, int slopeflag, int wetdry,
-                                                 const int* __restrict__ wd, const double* __restrict__ q,
-                                                 const double* __restrict__ mm, double* __restrict__ lam,
+                                                 const int* wd, const double* q,
+                                                 const double* mm, double* __restrict__ lam,
                                                  double* __restrict__ lb, double* __restrict__ g_hb) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = m.ne, np = m.np;
@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(128, 5) limit_vjp(const MeshView m, const Phys
 }
 
 // Per node: the cotangents of its bounds, summed over its star in star order.
-__global__ void node_bound_gather(const MeshView m, const double* __restrict__ lb, double* __restrict__ nb) {
+__global__ void node_bound_gather(const MeshView m, const double* lb, double* __restrict__ nb) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const int p0 = n < m.np ? m.star_ptr[n] : 0, p1 = n < m.np ? m.star_ptr[n + 1] : 0;
   chain_wait();
@@ -784,7 +784,7 @@ __global__ void node_bound_gather(const MeshView m, const double* __restrict__ l
 
 // Per element: the node-bound cotangents of the nodes whose min / max it
 // attains, added to its mean (mode 1) of that variable.
-__global__ void elem_bound_scatter(const MeshView m, const int* __restrict__ arg, const double* __restrict__ nb,
+__global__ void elem_bound_scatter(const MeshView m, const int* arg, const double* nb,
                                    double* __restrict__ lam) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = m.ne, np = m.np;
@@ -839,7 +839,7 @@ __global__ void ssp_adj(const __grid_constant__ SspAdjArgs A) {
   }
 }
 
-__global__ void gauge_eval(const double* __restrict__ q, int ne, const int* __restrict__ elem,
+__global__ void gauge_eval(const double* q, int ne, const int* __restrict__ elem,
                            const double* __restrict__ phi, int ng, double* __restrict__ eta) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   chain_wait();

@@ -219,7 +219,9 @@ __host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int 
 // each may start while the one before it ends.  Every thread passes chain_wait
 // before it reads or writes anything another kernel of the chain touches (what
 // comes before it reads only the mesh and the plan); chain_next lets the next
-// kernel's blocks in as this one's leave room.
+// kernel's blocks in as this one's leave room.  A buffer that a kernel of the
+// chain writes carries no const __restrict__ in another: its data changes while
+// that kernel, too, is already running.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Launches a kernel of the chain: it may start before the one
@@ -261,7 +263,7 @@ struct StageArgs {
   Physics ph;
   PhysF pf;  // ph rounded to FP32
   int irk;                                  // 1-based stage
-  const double* __restrict__ qin;           // state of stage irk (edges read it)
+  const double* qin;                        // state of stage irk (edges read it)
   double* qout;                             // state of stage irk+1
   const double* qhist[kMaxStages];          // state of stage I, I=1..irk
   const double* rhist[kMaxStages];          // RHS of stage I<irk (if needed)
@@ -269,7 +271,7 @@ struct StageArgs {
   double a[kMaxStages], b[kMaxStages];      // ATVD(irk,I), BTVD(irk,I)*DT
   int ssp;                                  // SspKind
   double ca0, ca, cb;
-  const int* __restrict__ wd;               // WDFLG (read)
+  const int* wd;                            // WDFLG (read)
   double timedg, rampdg;
   const double* __restrict__ ramp;          // RAMPDG of this stage in device memory (graph replays), or null: rampdg
   const double* __restrict__ ocean_zg;      // [(f*NEEDS + L)*2 + ipt] EMO*RFF*COS(ARGJ-EFA)
@@ -353,7 +355,7 @@ struct P2Args {
   Physics ph;
   PhysF pf;     // ph rounded to FP32 (mixed precision)
   int irk;
-  const double* __restrict__ qin;  // 18 rows (6*var + mode)
+  const double* qin;               // 18 rows (6*var + mode)
   double* qout;
   const double* qhist[kMaxStages];
   const double* rhist[kMaxStages];
@@ -397,8 +399,8 @@ DGSWEM_DECLARE_P2_LAUNCHERS(mixed_p2)
 struct AdjArgs {
   MeshView m;
   Physics ph;
-  const double* __restrict__ q;         // stage state at which L was evaluated
-  const double* __restrict__ nu;        // cotangent of L, 9*NE
+  const double* q;                      // stage state at which L was evaluated
+  const double* nu;                     // cotangent of L, 9*NE
   double* lam;                          // += (dL/dq)^T nu, 9*NE
   double* g_n;                          // += per element, or null (no Manning n)
   double* g_hb;                         // += [k*NE + e]
@@ -408,7 +410,7 @@ struct AdjArgs {
   double* eb;                           // 36*NE scratch: edge-point trace cotangents
   const int* __restrict__ edges;        // (element, local edge) pairs: interior edges from the in side, boundary edges
   int nedge;
-  const int* __restrict__ wd;           // WDFLG the stage kernel read (dry elements: no volume terms, dry-side edge rules)
+  const int* wd;                        // WDFLG the stage kernel read (dry elements: no volume terms, dry-side edge rules)
 };
 // One stage of the reverse SSP-RK accumulation: lam_I += a_I lam_j and
 // nu_I += b_I lam_j for I < n (b_I already times DT).
