@@ -26,8 +26,10 @@ void set_last_error(const std::string& msg) { g_last_error = msg; }
 #define DG_CUDA(call)                                                                     \
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess)                                                                \
+    if (e_ != cudaSuccess) {                                                              \
+      (void)cudaGetLastError(); /* reported here, not by the next launch's check */       \
       throw Failure(DGSWEM_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    }                                                                                     \
   } while (0)
 
 // p=1 basis at the quadrature, edge and corner points (orthogonal_basis_v1.F
@@ -272,8 +274,8 @@ struct DevBuf {
   }
   void alloc(size_t count) {
     release();
-    n = count;
     if (count) DG_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    n = count;
   }
   void ensure(size_t count) {  // grow only
     if (count > n) alloc(count);
@@ -545,10 +547,11 @@ struct LaunchTimer {
 
 unsigned grid_for(int n, int block) { return (unsigned)((n + block - 1) / block); }
 
-// Normals of the plan's edge tasks from the geometry table (device).
-void fill_task_normals(dgswem_cuda* h) {
+// Normals of a plan's edge tasks (the mesh view m's, ntile tiles) from the
+// geometry table, into out (device).
+void fill_task_normals(dgswem_cuda* h, const MeshView& m, unsigned ntile, double* out) {
   if (h->v2) return;
-  h->v->task_normals(h->mesh, kTileShapes[h->tile_shape].tile, h->tile_nrm.p, (unsigned)h->ntile, h->stream);
+  h->v->task_normals(m, kTileShapes[h->tile_shape].tile, out, ntile, h->stream);
   check_launch(h, "task_normals");
   --h->launches;  // part of the plan, not of a step
   DG_CUDA(cudaStreamSynchronize(h->stream));
@@ -565,7 +568,8 @@ void fill_task_normals(dgswem_cuda* h) {
 // mostly take one branch.  Tiles cover the first n_tiled elements (the owned
 // ones); `ne` is the row stride of link (all local elements, ghosts
 // included).  Tiles are planned in parallel (each writes only its own
-// elements' eslot).
+// elements' eslot).  The handle changes after the last call that can fail: a
+// plan that does not fit, or whose arrays do not, leaves it as it was.
 void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>& link,
                      const std::vector<unsigned>& einfo) {
   const TileShape shape = kTileShapes[h->tile_shape];
@@ -672,39 +676,49 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
     std::copy(ttasks[t].begin(), ttasks[t].end(), tasks.begin() + 2 * (size_t)t * max_tasks);
     std::copy(thalo[t].begin(), thalo[t].end(), halo.begin() + (size_t)t * max_halo);
   }
-  {
-    std::vector<int> order, rest;
-    for (int t = 0; t < ntile; ++t) {
-      bool interior = true;
-      for (int g : thalo[t]) interior = interior && g < n_tiled;
-      for (size_t i = 0; i < ttasks[t].size(); i += 2)
-        interior = interior && (ttasks[t][i] & 7u) != kIBarrier;
-      (interior ? order : rest).push_back(t);
-    }
-    h->n_tile_interior = (int)order.size();
-    order.insert(order.end(), rest.begin(), rest.end());
-    h->tile_order.upload(order.empty() ? std::vector<int>(1, 0) : order);
+  std::vector<int> order, rest;
+  for (int t = 0; t < ntile; ++t) {
+    bool interior = true;
+    for (int g : thalo[t]) interior = interior && g < n_tiled;
+    for (size_t i = 0; i < ttasks[t].size(); i += 2)
+      interior = interior && (ttasks[t][i] & 7u) != kIBarrier;
+    (interior ? order : rest).push_back(t);
   }
-  h->ntile = ntile;
-  h->tile_count.upload(count);
-  h->tile_tasks.upload(tasks);
-  h->tile_halo.upload(halo);
-  h->eslot.upload(eslot);
-  h->stage_smem = stage_smem;
-  MeshView& m = h->mesh;
+  const int n_interior = (int)order.size();
+  order.insert(order.end(), rest.begin(), rest.end());
+  DevBuf<int> d_order, d_count, d_halo;
+  DevBuf<unsigned> d_tasks, d_eslot;
+  DevBuf<double> d_nrm, d_xres;
+  d_order.upload(order.empty() ? std::vector<int>(1, 0) : order);
+  d_count.upload(count);
+  d_tasks.upload(tasks);
+  d_halo.upload(halo);
+  d_eslot.upload(eslot);
+  MeshView m = h->mesh;
   m.max_halo = max_halo;
   m.max_tasks = max_tasks;
   m.ne_tiled = n_tiled;
-  m.tile_count = reinterpret_cast<const int2*>(h->tile_count.p);
-  m.tile_tasks = reinterpret_cast<const uint2*>(h->tile_tasks.p);
-  m.tile_halo = h->tile_halo.p;
-  m.eslot = h->eslot.p;
+  m.tile_count = reinterpret_cast<const int2*>(d_count.p);
+  m.tile_tasks = reinterpret_cast<const uint2*>(d_tasks.p);
+  m.tile_halo = d_halo.p;
+  m.eslot = d_eslot.p;
   if (!h->v2) {
-    h->tile_nrm.alloc(2 * nt * max_tasks);
-    h->xres.alloc(6 * nt * max_tasks);
-    m.tile_nrm = h->tile_nrm.p;
-    if (m.egeo) fill_task_normals(h);  // a new plan of a built mesh
+    d_nrm.alloc(2 * nt * max_tasks);
+    d_xres.alloc(6 * nt * max_tasks);
+    m.tile_nrm = d_nrm.p;
+    if (m.egeo) fill_task_normals(h, m, (unsigned)ntile, d_nrm.p);  // a new plan of a built mesh
   }
+  h->mesh = m;
+  h->ntile = ntile;
+  h->n_tile_interior = n_interior;
+  h->stage_smem = stage_smem;
+  h->tile_order = std::move(d_order);
+  h->tile_count = std::move(d_count);
+  h->tile_tasks = std::move(d_tasks);
+  h->tile_halo = std::move(d_halo);
+  h->eslot = std::move(d_eslot);
+  h->tile_nrm = std::move(d_nrm);
+  h->xres = std::move(d_xres);
 }
 
 // Device element and node order: elements sorted along a Morton (Z-order)
@@ -993,7 +1007,7 @@ void build_layout(dgswem_cuda* h, const dgswem_cuda_setup* s, const PartPlan& pl
   m.ebht = h->ebht.p; m.ebcfsp = h->ebcfsp.p;
   m.ib_elem = h->ib_elem.p; m.ib_led = h->ib_led.p;
   m.ibht = h->ibht.p; m.ibcfsb = h->ibcfsb.p; m.ibcfsp = h->ibcfsp.p;
-  fill_task_normals(h);
+  fill_task_normals(h, m, (unsigned)h->ntile, h->tile_nrm.p);
 }
 
 // Halo index lists of a partitioned handle (local element ids), per kind,
@@ -2094,7 +2108,7 @@ namespace {
 
 // Rebuilds the stage tile plan for tile shape `shape` from the device copies
 // of the edge graph (link, einfo); on failure (the shape's plan does not fit
-// the task word or shared memory) the current plan stays.  Captured graphs
+// the task word, shared memory or device memory) the current plan stays.  Captured graphs
 // hold the old plan's launches: released.
 void replan(dgswem_cuda* h, int shape) {
   DG_CUDA(cudaStreamSynchronize(h->stream));
@@ -2108,7 +2122,7 @@ void replan(dgswem_cuda* h, int shape) {
   try {
     build_tile_plan(h, h->n_own, h->ne, link, info);
   } catch (...) {
-    h->tile_shape = old;  // the plan is uploaded only after every check passed
+    h->tile_shape = old;  // the handle kept the old shape's plan
     throw;
   }
 }
