@@ -863,6 +863,36 @@ __device__ __forceinline__ bool edge_task(const StageArgs& A, const real* tab, c
   return !ok;
 }
 
+// The terms of earlier stages in an SSP combination of any form, in their
+// order, into out (nine rows, row c at at(c)): term by term, the nine values of
+// a stage's state and right-hand side fetched together.  h0: the step-start
+// state, fetched by the caller where its coefficient is nonzero.  Bound by the
+// latency of those loads: value by value, each with its own loop over the
+// stages, a step of SSP(5,2) took 393 us on 200k elements (p=2: 916 us), this
+// way 187 (501); SSP(3,2), 132 -> 100.
+template <class Args, class At>
+__device__ __forceinline__ void ssp_history(const Args& A, At at, double h0[9], double out[9]) {
+#pragma unroll
+  for (int c = 0; c < 9; ++c) out[c] = 0.0;
+#pragma unroll 1
+  for (int I = 0; I < A.irk - 1; ++I) {
+    const double a = A.a[I], b = A.b[I];
+    double r[9];
+    if (I > 0 && a != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) h0[c] = A.qhist[I][at(c)];
+    if (b != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) r[c] = A.rhist[I][at(c)];
+    if (a != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) out[c] = madd(a, h0[c], out[c]);
+    if (b != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) out[c] = madd(b, r[c], out[c]);
+  }
+}
+
 // Phase 3 of the stage kernel: tile element el (global id e).
 // The sums are in the arithmetic type, the SSP combination in FP64 (in the
 // mixed variant: the RHS rounded to FP32, the stage states and their
@@ -988,7 +1018,7 @@ __device__ __forceinline__ void element_sums(const StageArgs& A, const real* tab
   // the compiler cannot reorder, nine round trips cost 70 us of 260 at 1M
   // elements; after the volume terms 3 us; prefetched before the edge sums 3 us)
   double h0[9];
-  if (A.ssp == kSspTwo)
+  if (A.irk > 1 && A.ca0 != 0.0)
 #pragma unroll
     for (int c = 0; c < 9; ++c) h0[c] = A.qhist[0][(size_t)c * ne + e];
   if (wde != 0) {
@@ -999,7 +1029,7 @@ __device__ __forceinline__ void element_sums(const StageArgs& A, const real* tab
   // SSP-RK combination (DG_hydro_timestep.F:238-290), zero coefficients
   // skipped: the stages whose nonzero terms are the current state and
   // right-hand side (the first), or those and the step-start state, without a
-  // branch per term
+  // branch per term; any other stage by ssp_history
   bool bad = false;
   double out[9];
   if (A.ssp != kSspAny) {
@@ -1011,16 +1041,13 @@ __device__ __forceinline__ void element_sums(const StageArgs& A, const real* tab
       out[c] = madd(A.cb, (double)rhs[c / 3][c % 3], acc);
     }
   } else {
+    ssp_history(A, [&](int c) { return (size_t)c * ne + e; }, h0, out);
+    if (A.ca != 0.0)
 #pragma unroll
-    for (int c = 0; c < 9; ++c) {
-      double acc = 0.0;
-      for (int I = 0; I < A.irk; ++I) {
-        const bool cur = I == A.irk - 1;
-        if (A.a[I] != 0.0) acc = acc + A.a[I] * (cur ? qs[el * kQStride + c] : A.qhist[I][(size_t)c * ne + e]);
-        if (A.b[I] != 0.0) acc = acc + A.b[I] * (cur ? (double)rhs[c / 3][c % 3] : A.rhist[I][(size_t)c * ne + e]);
-      }
-      out[c] = acc;
-    }
+      for (int c = 0; c < 9; ++c) out[c] = madd(A.ca, qs[el * kQStride + c], out[c]);
+    if (A.cb != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) out[c] = madd(A.cb, (double)rhs[c / 3][c % 3], out[c]);
   }
 #pragma unroll
   for (int c = 0; c < 9; ++c) {

@@ -871,9 +871,10 @@ __global__ void __launch_bounds__(kP2TileThreads, kP2Blocks) p2_tile(const __gri
   }
   // the SSP combination's step-start state, in one batch, behind the area sums
   double h0[9];
-  if (A.ssp == kSspTwo)
+  auto at = [&](int c) { return (size_t)(kP2Modes * (c / 3) + K0 + c % 3) * ne + e; };
+  if (A.irk > 1 && A.ca0 != 0.0)
 #pragma unroll
-    for (int c = 0; c < 9; ++c) h0[c] = A.qhist[0][(size_t)(kP2Modes * (c / 3) + K0 + c % 3) * ne + e];
+    for (int c = 0; c < 9; ++c) h0[c] = A.qhist[0][at(c)];
   const acc_t drdx = geo[EGeo::kDrdx * kP2Tile + el], dsdx = geo[EGeo::kDsdx * kP2Tile + el];
   const acc_t drdy = geo[EGeo::kDrdy * kP2Tile + el], dsdy = geo[EGeo::kDsdy * kP2Tile + el];
 #pragma unroll 1
@@ -902,36 +903,38 @@ __global__ void __launch_bounds__(kP2TileThreads, kP2Blocks) p2_tile(const __gri
   // SSP-RK combination (DG_hydro_timestep.F:238-290) in FP64
   double out[9];
   bool bad = false;
-#pragma unroll
-  for (int c = 0; c < 9; ++c) {
-    const int row = kP2Modes * (c / 3) + K0 + c % 3;
-    const size_t at = (size_t)row * ne + e;
+  auto current = [&](int c) {
 #ifdef DGSWEM_MIXED
-    const double qc = A.qin[at];
+    return A.qin[at(c)];
 #else
-    const double qc = qs[el * kP2SlotStride + row];  // the slot holds qin exactly
+    return qs[el * kP2SlotStride + kP2Modes * (c / 3) + K0 + c % 3];  // the slot holds qin exactly
 #endif
-    const double rk = (double)rhs[c / 3][c % 3];
-    double acc = 0.0;
-    if (A.ssp != kSspAny) {
+  };
+  if (A.ssp != kSspAny) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+      double acc = 0.0;
       if (A.ssp == kSspTwo) acc = madd(A.ca0, h0[c], acc);
-      acc = madd(A.ca, qc, acc);
-      acc = madd(A.cb, rk, acc);
-    } else {
-      for (int I = 0; I < A.irk; ++I) {
-        const bool cur = I == A.irk - 1;
-        if (A.a[I] != 0.0) acc = acc + A.a[I] * (cur ? qc : A.qhist[I][at]);
-        if (A.b[I] != 0.0) acc = acc + A.b[I] * (cur ? rk : A.rhist[I][at]);
-      }
+      acc = madd(A.ca, current(c), acc);
+      out[c] = madd(A.cb, (double)rhs[c / 3][c % 3], acc);
     }
-    out[c] = acc;
+  } else {
+    ssp_history(A, at, h0, out);
+    if (A.ca != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) out[c] = madd(A.ca, current(c), out[c]);
+    if (A.cb != 0.0)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) out[c] = madd(A.cb, (double)rhs[c / 3][c % 3], out[c]);
   }
 #pragma unroll
   for (int c = 0; c < 9; ++c) {
-    const size_t at = (size_t)(kP2Modes * (c / 3) + K0 + c % 3) * ne + e;
     bad = bad || isnan(out[c]);
-    A.qout[at] = out[c];
-    if (A.rout) A.rout[at] = (double)rhs[c / 3][c % 3];
+    A.qout[at(c)] = out[c];
+  }
+  if (A.rout) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) A.rout[at(c)] = (double)rhs[c / 3][c % 3];
   }
   if (bad) atomicOr(A.err, 1u);
 }
