@@ -703,8 +703,10 @@ void build_tile_plan(dgswem_cuda* h, int n_tiled, int ne, const std::vector<int>
   m.tile_halo = d_halo.p;
   m.eslot = d_eslot.p;
   if (!h->v2) {
-    d_nrm.alloc(2 * nt * max_tasks);
-    d_xres.alloc(6 * nt * max_tasks);
+    // two and six numbers a task, in the arithmetic type
+    const size_t pair = (2 * nt * max_tasks * h->v->real_bytes + sizeof(double) - 1) / sizeof(double);
+    d_nrm.alloc(pair);
+    d_xres.alloc(3 * pair);
     m.tile_nrm = d_nrm.p;
     if (m.egeo) fill_task_normals(h, m, (unsigned)ntile, d_nrm.p);  // a new plan of a built mesh
   }
