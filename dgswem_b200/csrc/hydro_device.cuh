@@ -224,6 +224,15 @@ __host__ __device__ inline StageLayout stage_layout(int tile, int max_halo, int 
 // that kernel, too, is already running.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Lets a kernel take all the dynamic shared memory a block can have.  The limit
+// is an attribute of the kernel on the device, shared by every handle and thread:
+// set before each launch (a host-side call, no device work), always to the same
+// value, so that no handle lowers it between another's call and launch.
+constexpr int kMaxBlockSmem = 227 * 1024;
+template <class K>
+void allow_block_smem(K* k) {
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+}
 // Launches a kernel of the chain: it may start before the one
 // ahead of it on the stream has ended.
 template <class... P, class... Args>

@@ -1023,7 +1023,7 @@ void launch_p2_stage(const P2Args& a, bool nonlin, cudaStream_t s) {
   if (a.ntile > 0) {  // the tile kernel
     const size_t smem = p2_layout(a.m.max_halo, a.m.max_tasks).bytes;
     auto* k = nonlin ? p2_tile<true> : p2_tile<false>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_block_smem(k);
     launch_chained(k, (unsigned)a.ntile, kP2TileThreads, smem, s, a);
     return;
   }
