@@ -70,17 +70,18 @@ STAGE_KERNEL_BYTES = 2.5 * 72 + 24 + 40 + 12 + 8 + 8
 # the whole RK stage adds the limiter's node ids 12 and the node min/max
 # written and read back 24
 STEP_BYTES_PER_ELEMENT_STAGE = STAGE_KERNEL_BYTES + 12 + 24
-# what stage_p1 reads beyond that model, per element-stage: the geometry rows
-# it copies to shared memory (normals, Jacobian terms, XLEN/AREAS, mean
-# Manning n: 112 B where the model counts 40 + 8), the tile plan (1.63 edge
-# tasks of 8 bytes and 0.25 halo ids per element on the Morton-ordered mesh)
-# and the packed edge kinds / task slots
-STAGE_OVERHEAD_BYTES = {"geometry_rows_beyond_model": 112 - 48, "tile_plan": 14, "edge_info": 8}
+# what stage_p1 reads beyond that model, per element-stage: the eight geometry
+# rows it copies to shared memory (inverse Jacobian, XLEN/AREAS, mean Manning n:
+# 64 B where the model counts 40 + 8), the tile plan (1.63 edge tasks, each a
+# word pair of 8 bytes and a normal of 16, and 0.25 halo ids of 4 bytes per
+# element on the Morton-ordered mesh) and the packed edge kinds / task slots
+STAGE_OVERHEAD_BYTES = {"geometry_rows_beyond_model": 64 - 48, "tile_plan": 1.63 * (8 + 16) + 0.25 * 4,
+                        "edge_info": 8}
 # DRAM bytes per element of one stage_p1 launch (strict build),
 # dram__bytes_read.sum + dram__bytes_write.sum from ncu on the same deck at
-# 999,192 elements: the mean of a stage-1 (270.9) and a stage-2 (346.5)
+# 999,192 elements: the mean of a stage-1 (270.4) and a stage-2 (343.3)
 # launch; traffic grows with the element count.
-STAGE_TRAFFIC_BYTES = 0.5 * (270.9 + 346.5)
+STAGE_TRAFFIC_BYTES = 0.5 * (270.4 + 343.3)
 
 
 def rank_env():

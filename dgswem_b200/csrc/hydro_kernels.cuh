@@ -462,19 +462,19 @@ __global__ void __launch_bounds__(128) ibarrier_sides(const __grid_constant__ St
 // kernel is bound by instruction issue: a finer split repeats the loads of an
 // element's modes, the task decode, the weights and the geometry for every
 // point and mode (4,670 thread instructions an element and stage in the first
-// stage, 1,550 of them FP64, against 2,270 and 1,180 here), and because the
+// stage, 1,550 of them FP64, against 2,135 and 1,185 here), and because the
 // values of one edge or element give straight-line code whose long dependent
 // chains (reciprocals, roots) the compiler interleaves: with a branch per
 // operation, as the operators' range checks make, a block of the kernel took
-// twice the cycles.  Three blocks of 128 threads with 168 registers and no
+// twice the cycles.  Three blocks of 128 threads with 158 registers and no
 // spills: four blocks of 128 registers, five of 96 and six of 80 spill and are
 // 11, 25 and 40 % slower.  On 1M elements (strict, wet/dry beach, mean of the
-// two stages) 245 us before, 144 us now.
+// two stages) 245 us before, 141.5 us now.
 // internal_edge_hydro.F, *_edge_hydro.F, rhs_dg_hydro.F, DG_hydro_timestep.F:238-290
 // ---------------------------------------------------------------------------
 
-// resident stage threads per SM the register allocation targets (FP64: 128
-// registers a thread); a shape of T threads per block is compiled for that
+// resident stage threads per SM the register allocation targets (FP64: at most
+// 168 registers a thread); a shape of T threads per block is compiled for that
 // many over T resident blocks
 #ifndef DGSWEM_STAGE_RESIDENT_THREADS
 #define DGSWEM_STAGE_RESIDENT_THREADS 384

@@ -440,12 +440,13 @@ __global__ void __launch_bounds__(128, 4) p2_elements(const __grid_constant__ P2
 //      the three variables in the order of p2_elements (boundary edges,
 //      interior edges as the slot sum, rain, area points), then the SSP
 //      combination.
-// Work is split so coarsely for the reasons given at stage_p1: 6,560 thread
-// instructions an element and stage (3,730 of them FP64) against 9,830 (3,840)
+// Work is split so coarsely for the reasons given at stage_p1: 6,530 thread
+// instructions an element and stage (3,620 of them FP64) against 9,830 (3,840)
 // by point and mode, the area and sum loops rolled (unrolled they cost 5 % in
-// instruction fetches).  250k elements, strict: 147.8 -> 129.6 us a stage, two
-// blocks of 218 registers an SM 133.6, four of 128 149; mixed, 130k elements:
-// 64.8 -> 50.1 us.
+// instruction fetches).  250k elements, strict: 147.8 -> 129.6 us a stage (two
+// blocks of 218 registers an SM 133.6, four of 128 149), 118.1 with the SSP
+// combination's long form out of the straight code (ssp_history); mixed, 130k
+// elements: 64.8 -> 46.1 us.
 // Each interior edge point is evaluated once per tile (twice for an edge
 // between tiles) and its flux stays in shared memory: no flux slots in HBM.
 // Every sum has p2_elements' operands and order, so both give the same bits.
